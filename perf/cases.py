@@ -128,7 +128,8 @@ def _sizes(case):
     return ps, qs, math.prod(ps), math.prod(qs)
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """X, the factors and Y (None without beta) as the call takes them."""
     ps, qs, K, L = _sizes(case)
     dt, M, batch = DTYPES[case["dt"]], case["M"], case["batch"]
     gen = torch.Generator(device="cuda").manual_seed(seed)
@@ -141,22 +142,28 @@ def prepare(case, seed):
             return torch.randn(*shape, dtype=dt, device="cuda", generator=gen)
         return uniform(*shape)
 
-    s = {"case": case, "ps": ps, "qs": qs}
     if case["call"] in ("gemkm", "gekmm"):
         left = case["call"] == "gekmm"
         xshape, zshape = ((K, M), (L, M)) if left else ((M, K), (M, L))
-        s["x"] = data(*xshape[::-1]).t() if case["tx"] else data(*xshape)
-        s["fs"] = []
+        x = data(*xshape[::-1]).t() if case["tx"] else data(*xshape)
+        fs = []
         for i, (p, q) in enumerate(zip(ps, qs)):
             r, c = (q, p) if left else (p, q)
             transposed = case["tf"] == "all" or (case["tf"] == "first" and i == 0)
-            s["fs"].append(uniform(c, r).t() if transposed else uniform(r, c))
-        s["y"] = data(*zshape) if case["beta"] != 0 else None
+            fs.append(uniform(c, r).t() if transposed else uniform(r, c))
+        return x, fs, data(*zshape) if case["beta"] != 0 else None
+    return data(batch, M, K), [uniform(batch, p, q) for p, q in zip(ps, qs)], None
+
+
+def prepare(case, seed):
+    ps, qs, K, L = _sizes(case)
+    dt, M, batch = DTYPES[case["dt"]], case["M"], case["batch"]
+    s = {"case": case, "ps": ps, "qs": qs}
+    s["x"], s["fs"], s["y"] = _inputs(case, seed)
+    if case["call"] in ("gemkm", "gekmm"):
         return s
     # what a program that calls a handle keeps: the handle, the result and the work buffers
     h = s["h"] = fastkron_b200.FastKron()
-    s["x"] = data(batch, M, K)
-    s["fs"] = [uniform(batch, p, q) for p, q in zip(ps, qs)]
     s["z"] = torch.empty(batch, M, L, dtype=dt, device="cuda")
     if case["call"] == "batched":
         _, te = h.sizes(M, ps, qs)
@@ -200,6 +207,33 @@ def work(case):
             cols = cols // p * q
             elems += M * cols
     return {"bytes": case["batch"] * elems * es, "flops": case["batch"] * 2 * M * macs}
+
+
+def exact(case, seed):
+    """What run returns, in 64-bit arithmetic: the factors from the last to the first, each contracting the
+    fastest index and putting its own in front of the others (after all of them the order is the original)."""
+    x, fs, y = _inputs(case, seed)
+    left = case["call"] == "gekmm"
+    if left:
+        x, fs = x.t(), [f.t() for f in fs]
+    t = x.double()
+    if t.dim() == 2:
+        t, fs = t[None], [f[None] if f.dim() == 2 else f for f in fs]
+    batch, M = t.shape[:2]
+    steps = []
+    for f in reversed(fs):
+        p = f.shape[1]
+        t = torch.matmul(t.reshape(batch, -1, p), f.double())                     # [batch][M * S][Q]
+        t = t.reshape(batch, M, -1, f.shape[2]).transpose(2, 3).reshape(batch, M, -1)
+        if case["call"] == "forward":
+            steps.append(t)
+    if case["call"] == "forward":
+        return [steps[-1]] + [u.reshape(-1) for u in steps[-2::-1]]
+    if case["call"] == "batched":
+        return t
+    z = t[0].t() if left else t[0]
+    z = case["alpha"] * z
+    return z if y is None else z + case["beta"] * y.double()
 
 
 def tolerance(case):
