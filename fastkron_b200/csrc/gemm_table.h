@@ -36,4 +36,12 @@ inline bool gemmAnyEligible(uint32_t P, uint32_t Q) {
   return (uint64_t)P * Q >= 64 || (P >= 5 && Q >= 5);
 }
 
+// The split tensor-core kernel (kernel_gemm_split.cu), fp32: factors up to 128 on either side; `total` is the
+// number of positions (rows of the contraction).  Smaller factors leave the FMA kernels bound by memory already
+// (256 rows, 24x24 three times: 58 us, against 78 us with the split kernel's fixed work per position), and below 1024
+// positions the eight tiles of 128 leave most of the chip idle.
+inline bool gemmSplitEligible(uint32_t P, uint32_t Q, uint64_t total) {
+  return P >= 17 && Q >= 17 && P <= 128 && Q <= 128 && P * Q >= 1024 && total >= 1024 && total < (1ull << 31);
+}
+
 }  // namespace fkb

@@ -96,8 +96,13 @@ static fastKronError launchGemmOne(const Pass& ps, const LaunchCtx& cx, int mode
 // and stays scalar.
 static fastKronError launchGemmFixed(const Pass& ps, const LaunchCtx& cx);
 
-// The fixed-shape kernels where they apply, the any-shape kernel otherwise.
+// The split tensor-core kernel where its rule admits the pass, the fixed-shape FMA kernels where they
+// apply, the any-shape kernel otherwise.
 fastKronError launchGemm(const Pass& ps, const LaunchCtx& cx) {
+  if (!cx.tf32) {
+    const fastKronError e = launchGemmSplit(ps, cx);
+    if (e != fastKronKernelNotFound) return e;
+  }
   if (ps.variant != 3) {
     const fastKronError e = launchGemmFixed(ps, cx);
     if (e != fastKronKernelNotFound) return e;

@@ -1,0 +1,155 @@
+"""The split tensor-core pass (csrc/kernel_gemm_split.cu) at the sizes where it can go wrong: partial tiles, remainders of 16 and 32, both orientations, operands that are not
+16-byte aligned, beta*Y in place of the result, values that a bf16 split cannot hold.
+
+Bound.  One step of P products in precision u errs by at most (P + 2) u of the sum of the products' magnitudes
+(one rounding per product for an FMA chain; for the split pass one accumulator rounding, of at most 2 u, per 16
+products of each of its six terms, and 2^-26 for the terms it leaves out).  Over the steps the bounds add up, and
+alpha and beta*Y add two roundings: |error| <= u * (sum (P_i + 4) + 4) * (|alpha| |X| |F| + |beta| |Y|)."""
+import ctypes
+import os
+import sys
+
+import numpy as np
+import pytest
+
+sys.path.insert(0, os.path.dirname(os.path.abspath(__file__)))
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    from fastkron_b200 import lib as fk
+    L = fk.get()
+    L.fkbGemmSplitLaunches.restype = ctypes.c_ulonglong
+    L.fkbLaunchCount.restype = ctypes.c_ulonglong
+    yield L
+    assert L.fkbGemmSplitTimeouts() == 0
+
+
+def product(x, fs):
+    t = x
+    for f in reversed(fs):
+        p, q = f.shape
+        t = t.reshape(t.shape[0], -1, p) @ f
+        t = t.swapaxes(1, 2).reshape(t.shape[0], -1)
+    return t
+
+
+def check(z, x, fs, alpha, beta, y, u):
+    want = alpha * product(x, fs)
+    mag = abs(alpha) * product(np.abs(x), [np.abs(f) for f in fs])
+    if beta:
+        want = want + beta * y
+        mag = mag + abs(beta) * np.abs(y)
+    bound = u * (sum(f.shape[0] + 4 for f in fs) + 4) * mag
+    assert np.all(np.abs(z - want) <= bound), np.max(np.abs(z - want) / np.maximum(bound, 1e-300))
+
+
+def call(mm, dt, M, ps, qs, tx, tf, beta, shift, seed=0):
+    """Runs the front-end on operands `shift` elements off their allocation; returns z and the operands as
+    float64 MKM matrices."""
+    import torch
+    import fastkron_b200
+    rng = np.random.default_rng(seed)
+    tdt = torch.float32 if dt == "f32" else torch.float64
+
+    def dev(a):
+        buf = torch.empty(a.size + shift, dtype=tdt, device="cuda")
+        v = buf[shift:].view(*a.shape)
+        v.copy_(torch.from_numpy(np.ascontiguousarray(a)))
+        return v
+
+    ndt = np.float32 if dt == "f32" else np.float64
+    K, L = int(np.prod(ps)), int(np.prod(qs))
+    x = rng.uniform(-1, 1, (M, K)).astype(ndt)
+    fs = [rng.uniform(-1, 1, (p, q)).astype(ndt) for p, q in zip(ps, qs)]
+    y = rng.uniform(-1, 1, (M, L)).astype(ndt)
+    xm, fm, ym = (x, fs, y) if mm == "mkm" else (x.T, [f.T for f in fs], y.T)
+    xd = dev(xm.T).t() if tx else dev(xm)
+    fd = [dev(f.T).t() if tf else dev(f) for f in fm]
+    yd = dev(ym) if beta else None
+    if mm == "mkm":
+        z = fastkron_b200.gemkm(xd, fd, 2.0 if beta else 1.0, beta, yd)
+    else:
+        z = fastkron_b200.gekmm(fd, xd, 2.0 if beta else 1.0, beta, yd)
+    z = z.cpu().numpy().astype(np.float64)
+    d = lambda a: a.astype(np.float64)
+    return (z if mm == "mkm" else z.T), d(x), [d(f) for f in fs], d(y)
+
+
+SPLIT = [
+    # M, ps, qs
+    (128, [33, 17], [32, 61]), (40, [64, 64], [64, 64]), (9, [127, 128], [128, 127]), (33, [128, 40], [96, 128]),
+    (17, [65, 80], [113, 49]), (20, [48, 112], [112, 48]), (1, [64, 33, 34], [33, 64, 36]), (300, [128, 128], [128, 128]),
+]
+
+
+@pytest.mark.parametrize("mm,tx,tf,beta,shift", [("mkm", 0, 0, 0.0, 0), ("mkm", 1, 1, 1.0, 0), ("kmm", 0, 0, -0.5, 0),
+                                                 ("kmm", 1, 0, 0.0, 0), ("mkm", 0, 1, 1.0, 1), ("kmm", 0, 0, 0.0, 3)])
+@pytest.mark.parametrize("M,ps,qs", SPLIT, ids=lambda v: str(v).replace(" ", ""))
+def test_split_pass(lib, M, ps, qs, mm, tx, tf, beta, shift):
+    n0 = lib.fkbGemmSplitLaunches()
+    z, x, fs, y = call(mm, "f32", M, ps, qs, tx, tf, beta, shift)
+    assert lib.fkbGemmSplitLaunches() > n0, "the split kernel did not run"
+    check(z, x, fs, 2.0 if beta else 1.0, beta, y, 2.0 ** -24)
+
+
+def test_split_forward_layout(lib):
+    """The forward variants' rotating layout: contraction index contiguous in, position index contiguous out."""
+    import torch
+    import fastkron_b200
+    h = fastkron_b200.FastKron()
+    M, ps, qs = 37, [33, 64], [40, 127]
+    x = torch.rand(M, 33 * 64, device="cuda") - 0.5
+    fs = [torch.rand(p, q, device="cuda") - 0.5 for p, q in zip(ps, qs)]
+    ye, ie = h.sizes_forward(M, ps, qs)
+    z, inter = torch.empty(ye, device="cuda"), [torch.empty(n, device="cuda") for n in ie]
+    n0 = lib.fkbGemmSplitLaunches()
+    h.raw_forward("mkm", "s", M, ps, qs, x.data_ptr(), 1, [f.data_ptr() for f in fs], 1, z.data_ptr(), [t.data_ptr() for t in inter])
+    assert lib.fkbGemmSplitLaunches() == n0 + 2
+    xn, fn = x.cpu().numpy().astype(np.float64), [f.cpu().numpy().astype(np.float64) for f in fs]
+    check(z.view(M, -1).cpu().numpy(), xn, fn, 1.0, 0.0, None, 2.0 ** -24)
+    t = xn.reshape(M, 33, 64) @ fn[1]
+    t = t.swapaxes(1, 2).reshape(M, -1)
+    err = np.abs(inter[0].view(M, -1).cpu().numpy() - t)
+    mag = (np.abs(xn).reshape(M, 33, 64) @ np.abs(fn[1])).swapaxes(1, 2).reshape(M, -1)
+    assert np.all(err <= 2.0 ** -24 * 72 * mag)
+    h.close()
+
+
+@pytest.mark.parametrize("where", ["x", "f"])
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.4e38, -1.8e38, 1e-38, 1e-42, 2e-28, 0.0])
+def test_split_pass_on_values_a_bf16_split_cannot_hold(lib, where, value):
+    """Same result as the FMA kernels where those give inf or NaN; rows and factor columns of tiny magnitude keep
+    their relative precision."""
+    import torch
+    import fastkron_b200
+    torch.manual_seed(1)
+    M, P, Q = 2000, 64, 50
+    x, f = torch.rand(M, P, device="cuda") - 0.5, torch.rand(P, Q, device="cuda") - 0.5
+    if where == "x":
+        if 0 < abs(value) < 1:
+            x[77] *= value                       # a whole row
+            x[1999] = 0
+        else:
+            x[77, 5] = value
+            x[1999, 63] = value
+    elif 0 < abs(value) < 1:
+        f[:, 7] *= value
+    else:
+        f[9, 7] = value
+    n0 = lib.fkbGemmSplitLaunches()
+    z = fastkron_b200.gemkm(x, [f]).cpu().numpy().astype(np.float64)
+    assert lib.fkbGemmSplitLaunches() == n0 + 1
+    lib.fkbSetSplitOff(1)
+    w = fastkron_b200.gemkm(x, [f]).cpu().numpy().astype(np.float64)
+    lib.fkbSetSplitOff(0)
+    assert np.array_equal(np.isnan(z), np.isnan(w))
+    assert np.array_equal(np.isinf(z), np.isinf(w)) and np.array_equal(z[np.isinf(z)], w[np.isinf(w)])
+    xn, fn = x.cpu().numpy().astype(np.float64), f.cpu().numpy().astype(np.float64)
+    ok = np.isfinite(w)
+    with np.errstate(invalid="ignore", over="ignore"):
+        want, mag = xn @ fn, np.abs(xn) @ np.abs(fn)
+    # 2^-149: the spacing of denormal results, once per product
+    assert np.all((np.abs(z - want) <= 2.0 ** -24 * (P + 8) * mag + P * 2.0 ** -149)[ok])
