@@ -202,7 +202,7 @@ def time_config(h, c, steps, warmup, profile=False):
         passes = []
         for p in range(per):
             vals = [ms[s * per + p] for s in range(steps)]
-            passes.append({"kind": ["generic", "tile", "gemm"][kinds[p]], "ms": float(np.mean(vals))})
+            passes.append({"kind": ["generic", "tile", "gemm", "chain"][kinds[p]], "ms": float(np.mean(vals))})
     total_ms = float(sum(times))
     return {"ms_per_step": total_ms / steps, "ms_min": float(min(times)), "launches": int(launches),
             "passes": passes, "buffers": (x, fs, y, z, t1, t2)}

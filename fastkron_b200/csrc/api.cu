@@ -297,11 +297,11 @@ void fkbSetForceGeneric(int on) { setForceGenericOverride(on != 0); }
 void fkbSetAnyMinElems(int elems) { gAnyMinElems = elems > 0 ? elems : 0; }
 
 // ---- introspection used by the host-side tests (not part of the reference ABI) --
-// Writes the textual plan of a problem into buf; returns the number of passes
+// Writes the textual plan of a problem, or the launches it is regrouped into, into buf; returns their number
 // or a negative fastKronError.
-int fkbDescribePlan(int isKmm, int isDouble, uint32_t M, uint32_t N, const uint32_t* Ps,
-                    const uint32_t* Qs, int opX, int opF, int forwardMode, int haveTemp2, int fusion,
-                    int align, char* buf, size_t bufLen) {
+static int describeProblem(bool launches, int isKmm, int isDouble, uint32_t M, uint32_t N, const uint32_t* Ps,
+                           const uint32_t* Qs, int opX, int opF, int forwardMode, int haveTemp2, int fusion,
+                           int align, char* buf, size_t bufLen) {
   Problem pr;
   if (!fillProblem(&pr, isKmm ? MMType::KMM : MMType::MKM, isDouble ? DType::F64 : DType::F32, M, N,
                    Ps, Qs, (fastKronOp)opX, (fastKronOp)opF))
@@ -316,6 +316,7 @@ int fkbDescribePlan(int isKmm, int isDouble, uint32_t M, uint32_t N, const uint3
   Plan plan;
   fastKronError e = makePlan(pr, po, &plan);
   if (e != fastKronSuccess) return -(int)e;
+  if (launches) fuseLaunches(pr, po, &plan);
   const std::string s = plan.describe();
   if (buf && bufLen) {
     const size_t n = s.size() < bufLen - 1 ? s.size() : bufLen - 1;
@@ -323,6 +324,17 @@ int fkbDescribePlan(int isKmm, int isDouble, uint32_t M, uint32_t N, const uint3
     buf[n] = 0;
   }
   return (int)plan.passes.size();
+}
+
+int fkbDescribePlan(int isKmm, int isDouble, uint32_t M, uint32_t N, const uint32_t* Ps, const uint32_t* Qs, int opX,
+                    int opF, int forwardMode, int haveTemp2, int fusion, int align, char* buf, size_t bufLen) {
+  return describeProblem(false, isKmm, isDouble, M, N, Ps, Qs, opX, opF, forwardMode, haveTemp2, fusion, align, buf, bufLen);
+}
+
+// The same for the launches of one (unbatched) call: what Engine::run makes of the plan.
+int fkbDescribeLaunches(int isKmm, int isDouble, uint32_t M, uint32_t N, const uint32_t* Ps, const uint32_t* Qs, int opX,
+                        int opF, int forwardMode, int haveTemp2, int fusion, int align, char* buf, size_t bufLen) {
+  return describeProblem(true, isKmm, isDouble, M, N, Ps, Qs, opX, opF, forwardMode, haveTemp2, fusion, align, buf, bufLen);
 }
 
 }  // extern "C"

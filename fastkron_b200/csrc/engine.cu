@@ -168,6 +168,7 @@ fastKronError Engine::run(Problem pr, const CallOperands& ops) {
     Plan plan;
     fastKronError e = makePlan(pr, po, &plan);
     if (e != fastKronSuccess) return e;
+    fuseLaunches(pr, po, &plan);
     // fastKronOptionsTune: time candidate plans once on the caller's own buffers (X and the
     // factors are never written; Z and the temporaries are scratch until the real run) and keep
     // the fastest.  Candidates: the table's plan, the unfused plan, and every distinct plan that
@@ -184,6 +185,7 @@ fastKronError Engine::run(Problem pr, const CallOperands& ops) {
         alt.maxFuse = cap;
         Plan other;
         if (makePlan(pr, alt, &other) != fastKronSuccess) continue;
+        fuseLaunches(pr, alt, &other);
         const std::string d = other.describe();
         bool dup = false;
         for (const std::string& s2 : seen) dup = dup || s2 == d;
@@ -272,6 +274,7 @@ fastKronError Engine::launchPass(const Pass& ps, const LaunchCtx& cx) {
   fastKronError e = fastKronKernelNotFound;
   if (ps.kind == KernelKind::Tile) e = launchTile(ps, cx);
   else if (ps.kind == KernelKind::Gemm) e = launchGemm(ps, cx);
+  else if (ps.kind == KernelKind::Chain) e = launchChain(ps, cx);
   if (e == fastKronKernelNotFound && ps.nf == 1) { e = launchGeneric(ps, cx); ranKind = (int)KernelKind::Generic; }
   if (evEnd) { cudaEventRecord(evEnd, stream); evKinds_.push_back(ranKind); }
   if (e != fastKronSuccess) return e;
@@ -309,6 +312,7 @@ fastKronError Engine::execute(const Problem& pr, const Plan& plan, const CallOpe
     cx.tf32 = tf32Mode();
     for (int k = 0; k < ps.nf; k++) cx.F[k] = ops.Fs[ps.f0 + k];
     factorStrides(pr.mm, pr.opF, ps.P[0], ps.Q[0], &cx.fsP, &cx.fsQ);
+    cx.fPMajor = factorPMajor(pr.mm, pr.opF);
     if (batch > 1) {
       // element distance between the batch entries of a logical buffer
       auto strideOf = [&](Buf b) -> uint64_t {

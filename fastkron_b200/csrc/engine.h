@@ -103,9 +103,9 @@ class Engine {
 };
 
 // Factor element strides for (mm, opF): element (p,q) at p*fsP + q*fsQ.
+inline bool factorPMajor(MMType mm, fastKronOp opF) { return (mm == MMType::MKM) ? (opF == fastKronOp_N) : (opF == fastKronOp_T); }
 inline void factorStrides(MMType mm, fastKronOp opF, uint32_t P, uint32_t Q, int64_t* fsP, int64_t* fsQ) {
-  const bool pMajor = (mm == MMType::MKM) ? (opF == fastKronOp_N) : (opF == fastKronOp_T);
-  if (pMajor) { *fsP = Q; *fsQ = 1; } else { *fsP = 1; *fsQ = P; }
+  if (factorPMajor(mm, opF)) { *fsP = Q; *fsQ = 1; } else { *fsP = 1; *fsQ = P; }
 }
 
 }  // namespace fkb

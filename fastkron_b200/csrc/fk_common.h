@@ -24,7 +24,8 @@ inline size_t dtypeSize(DType t) { return t == DType::F32 ? 4 : 8; }
 enum class KernelKind : int {
   Generic = 0,   // one thread per output element, arbitrary strides, any P/Q
   Tile    = 1,   // small power-of-two square factors fused in shared memory
-  Gemm    = 2    // large factors, register-blocked FFMA/DFMA contraction
+  Gemm    = 2,   // large factors, register-blocked FFMA/DFMA contraction
+  Chain   = 3    // several consecutive factors of any shape in one launch
 };
 
 // Logical buffer ids a pass reads from / writes to.
@@ -102,6 +103,9 @@ struct PlanOptions {
 
 // Build the list of passes for a problem.  Pure host code.
 fastKronError makePlan(const Problem& pr, const PlanOptions& opt, Plan* out);
+// The launches of a plan: runs of single-factor passes on factors of any shape are regrouped so that several
+// factors share a launch (KernelKind::Chain).  What Engine::run executes; pure host code.
+void fuseLaunches(const Problem& pr, const PlanOptions& opt, Plan* plan);
 // Process-wide cap on the fusion depth (the offline tuner's hook; 0 = none).
 void setMaxFuseOverride(int cap);
 // Process-wide "every pass on the one-thread-per-output kernel" (measurement / cross-check hook).

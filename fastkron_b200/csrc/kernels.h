@@ -28,7 +28,8 @@ struct LaunchCtx {
   void*       dst = nullptr;      // pass output
   const void* Y   = nullptr;      // epilogue operand (may be null when beta == 0)
   const void* F[kMaxGroup] = {nullptr};   // device pointers of factors f0 .. f0+nf-1
-  int64_t fsP = 1, fsQ = 1;       // factor element (p,q) at p*fsP + q*fsQ
+  int64_t fsP = 1, fsQ = 1;       // factor element (p,q) at p*fsP + q*fsQ (of the pass's first factor)
+  bool fPMajor = true;            // every factor stored as [p][q] (q contiguous); else [q][p]
   double alpha = 1.0, beta = 0.0; // applied only when pass.epilogue
   int smCount = 148;
   Scatter scatter;                // only honoured by the Generic and Gemm launchers
@@ -49,7 +50,7 @@ struct LaunchCtx {
 
 // True when the kernel that runs `ps` takes a strided batch in one launch.
 inline bool passBatchCapable(const Pass& ps) {
-  if (ps.kind == KernelKind::Generic) return true;
+  if (ps.kind == KernelKind::Generic || ps.kind == KernelKind::Chain) return true;
   if (ps.kind == KernelKind::Gemm) return ps.variant == 3;
   return ps.kind == KernelKind::Tile && ps.variant == 0;
 }
@@ -58,6 +59,7 @@ inline bool passBatchCapable(const Pass& ps) {
 // family (the caller then falls back to the generic kernel), or a CUDA failure
 // mapped to a fastKronError.
 fastKronError launchGeneric(const Pass& ps, const LaunchCtx& cx);
+fastKronError launchChain(const Pass& ps, const LaunchCtx& cx);
 fastKronError launchTile(const Pass& ps, const LaunchCtx& cx);
 fastKronError launchGemm(const Pass& ps, const LaunchCtx& cx);
 fastKronError launchGemmTf32(const Pass& ps, const LaunchCtx& cx);   // only reached through launchGemm

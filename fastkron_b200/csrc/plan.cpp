@@ -20,6 +20,7 @@
 #include "tile_table.h"
 #include "gemm_table.h"
 #include "tile_db.h"
+#include "chain_table.h"
 
 #include <sstream>
 #include <stdlib.h>
@@ -92,6 +93,30 @@ static TileChoice chooseTile(DType dt, uint32_t P, int avail, uint64_t B, bool f
     if (even >= 1 && even < c.nf) c.nf = even;
   }
   return c;
+}
+
+// Source and destination of every pass, by the rules at the head of the file.
+static void assignBuffers(const Problem& pr, const PlanOptions& opt, Plan* out) {
+  const size_t n = out->passes.size();
+  out->usesT2 = false;
+  for (size_t k = 0; k < n; k++) {
+    Pass& ps = out->passes[k];
+    const bool last = (k + 1 == n);
+    ps.epilogue = last;
+    if (pr.forward) {
+      ps.src = (k == 0) ? Buf::X : out->passes[k - 1].dst;
+      // the pass consuming factor f writes Intermediates[f-1]; the last writes Z
+      ps.dst = last ? Buf::Z : (Buf)((int)Buf::I0 + (ps.f0 - 1));
+      continue;
+    }
+    Buf seq[2];
+    if (opt.haveT2) { seq[0] = Buf::T1; seq[1] = Buf::T2; }
+    else if (n % 2 == 1) { seq[0] = Buf::Z; seq[1] = Buf::T1; }
+    else { seq[0] = Buf::T1; seq[1] = Buf::Z; }
+    ps.src = (k == 0) ? Buf::X : out->passes[k - 1].dst;
+    ps.dst = last ? Buf::Z : seq[k & 1];
+    if (!last && (ps.dst == Buf::T2 || ps.dst == Buf::Z)) out->usesT2 = true;
+  }
 }
 
 fastKronError makePlan(const Problem& pr, const PlanOptions& optIn, Plan* out) {
@@ -215,33 +240,101 @@ fastKronError makePlan(const Problem& pr, const PlanOptions& optIn, Plan* out) {
     i -= ps.nf;
   }
 
-  // ---- buffer assignment -------------------------------------------------
-  const size_t n = out->passes.size();
-  out->usesT2 = false;
-  for (size_t k = 0; k < n; k++) {
-    Pass& ps = out->passes[k];
-    const bool last = (k + 1 == n);
-    ps.epilogue = last;
-    if (pr.forward) {
-      ps.src = (k == 0) ? Buf::X : out->passes[k - 1].dst;
-      // the pass consuming factor f writes Intermediates[f-1]; the last writes Z
-      ps.dst = last ? Buf::Z : (Buf)((int)Buf::I0 + (ps.f0 - 1));
-      continue;
-    }
-    Buf seq[2];
-    if (opt.haveT2) { seq[0] = Buf::T1; seq[1] = Buf::T2; }
-    else if (n % 2 == 1) { seq[0] = Buf::Z; seq[1] = Buf::T1; }
-    else { seq[0] = Buf::T1; seq[1] = Buf::Z; }
-    ps.src = (k == 0) ? Buf::X : out->passes[k - 1].dst;
-    ps.dst = last ? Buf::Z : seq[k & 1];
-    if (!last && (ps.dst == Buf::T2 || ps.dst == Buf::Z)) out->usesT2 = true;
-  }
+  assignBuffers(pr, opt, out);
   return fastKronSuccess;
+}
+
+// ---- launches -----------------------------------------------------------------------------
+
+// A factor whose single-factor pass may share a launch with its neighbours.  Larger fp32 factors belong to the
+// split tensor-core kernel, larger fp64 ones fill a tile with a single factor.
+static bool chainable(const Problem& pr, const Pass& ps) {
+  if (ps.nf != 1 || (ps.kind != KernelKind::Generic && ps.kind != KernelKind::Gemm)) return false;
+  const uint32_t most = pr.dt == DType::F32 ? 32 : 64;
+  return ps.P[0] <= most && ps.Q[0] <= most;
+}
+
+// Factors f0 .. f1 as one pass.
+static Pass groupPass(const Problem& pr, int f0, int f1) {
+  Pass ps;
+  ps.kind = KernelKind::Chain;
+  ps.f0 = f0; ps.nf = f1 - f0 + 1;
+  uint64_t Pg = 1, Qg = 1, A = 1, B = 1;
+  for (int k = 0; k < ps.nf; k++) { ps.P[k] = pr.P[f0 + k]; ps.Q[k] = pr.Q[f0 + k]; Pg *= ps.P[k]; Qg *= ps.Q[k]; }
+  for (int j = 0; j < f0; j++) A *= pr.P[j];
+  for (uint32_t j = (uint32_t)f1 + 1; j < pr.N; j++) B *= pr.Q[j];
+  const Layout cur = f1 + 1 == (int)pr.N ? inputLayout(pr) : matLayout(pr, A * Pg * B);
+  const Layout nxt = matLayout(pr, A * Qg * B);
+  ps.M = pr.M; ps.A = A; ps.B = B;
+  ps.xsM = cur.ms; ps.xsB = cur.cs; ps.xsG = (int64_t)B * cur.cs; ps.xsA = (int64_t)(Pg * B) * cur.cs;
+  ps.zsM = nxt.ms; ps.zsB = nxt.cs; ps.zsG = (int64_t)B * nxt.cs; ps.zsA = (int64_t)(Qg * B) * nxt.cs;
+  if (cur.cs != 1 && nxt.cs != 1) {                  // m is the fastest index on both sides: fold it into B
+    ps.M = 1; ps.B = B * pr.M;
+    ps.xsM = ps.zsM = 0; ps.xsB = ps.zsB = 1;
+    ps.xsG = ps.zsG = (int64_t)ps.B;
+    ps.xsA = (int64_t)(Pg * ps.B); ps.zsA = (int64_t)(Qg * ps.B);
+  }
+  return ps;
+}
+
+// Estimated device time (us) of factors f0 .. f1 in one launch; negative when they do not fit.
+static double groupCost(const Problem& pr, int f0, int f1) {
+  const Pass ps = groupPass(pr, f0, f1);
+  const double es = (double)dtypeSize(pr.dt), pos = (double)ps.M * ps.A * ps.B;
+  const double bytes = pos * ((double)ps.Pg() + (double)ps.Qg()) * es;
+  if (pos >= 2147483648.0) return -1;
+  if (f0 == f1) return 3 + bytes / 3.0e6;            // the single-factor kernels
+  ChainShape s;
+  if (!chainShape(pr.dt, ps.nf, ps.P, ps.Q, ps.xsG == 1 || ps.zsG == 1, (uint64_t)pos, &s)) return -1;
+  // short runs of a strided side cost sectors
+  double runs = 1;
+  if (ps.xsG != 1 || ps.zsG != 1) { const double run = s.W * es; runs = run >= 64 ? 1 : run >= 32 ? 1.3 : 1.8; }
+  if (s.smem > kChainSmem3) runs *= 1.15;
+  return 3 + bytes / 5.0e6 * runs;
+}
+
+void fuseLaunches(const Problem& pr, const PlanOptions& opt, Plan* plan) {
+  // strided batches and the forward variants keep one launch per pass
+  if (pr.batch > 1 || pr.forward || !opt.fusion || opt.forceGeneric || gForceGeneric || opt.isolateFirst) return;
+  int most = kMaxGroup;
+  if (opt.maxFuse > 0 && opt.maxFuse < most) most = opt.maxFuse;
+  if (gMaxFuseOverride > 0 && gMaxFuseOverride < most) most = gMaxFuseOverride;
+  std::vector<Pass> out;
+  const std::vector<Pass>& in = plan->passes;
+  for (size_t k = 0; k < in.size();) {
+    size_t e = k;
+    while (e < in.size() && chainable(pr, in[e])) e++;
+    const int n = (int)(e - k);
+    if (n < 2) { out.push_back(in[k]); k++; continue; }
+    // cheapest split of the run into groups: best[c] covers its first c passes
+    std::vector<double> best(n + 1, 1e30);
+    std::vector<int> from(n + 1, 0);
+    best[0] = 0;
+    for (int c = 1; c <= n; c++)
+      for (int g = 1; g <= most && g <= c; g++) {
+        const double t = groupCost(pr, in[k + c - 1].f0, in[k + c - g].f0);
+        if (t >= 0 && best[c - g] + t < best[c]) { best[c] = best[c - g] + t; from[c] = c - g; }
+      }
+    if (best[n] >= 1e30) { out.insert(out.end(), in.begin() + k, in.begin() + e); k = e; continue; }
+    std::vector<Pass> rev;
+    for (int c = n; c > 0; c = from[c])
+      rev.push_back(c - from[c] == 1 ? in[k + c - 1] : groupPass(pr, in[k + c - 1].f0, in[k + from[c]].f0));
+    out.insert(out.end(), rev.rbegin(), rev.rend());
+    k = e;
+  }
+  Plan fused;
+  fused.passes = out;
+  assignBuffers(pr, opt, &fused);
+  // without temp2 the result doubles as scratch; regrouping must not put a matrix wider than it there
+  if (!opt.haveT2)
+    for (const Pass& ps : fused.passes)
+      if (!ps.epilogue && ps.dst == Buf::Z && ps.A * ps.Qg() * ps.B * ps.M > (uint64_t)pr.M * pr.L()) return;
+  *plan = fused;
 }
 
 std::string Plan::describe() const {
   std::ostringstream os;
-  static const char* kn[] = {"generic", "tile", "gemm"};
+  static const char* kn[] = {"generic", "tile", "gemm", "chain"};
   auto bn = [](Buf b) -> std::string {
     switch (b) { case Buf::X: return "X"; case Buf::T1: return "T1"; case Buf::T2: return "T2";
                  case Buf::Z: return "Z"; default: return "I" + std::to_string((int)b - (int)Buf::I0); }

@@ -1,4 +1,5 @@
-"""The split tensor-core pass (csrc/kernel_gemm_split.cu) at the sizes where it can go wrong: partial tiles, remainders of 16 and 32, both orientations, operands that are not
+"""The split tensor-core pass (csrc/kernel_gemm_split.cu) and the chain launches (csrc/kernel_chain.cu) at the
+sizes where they can go wrong: partial tiles, remainders of 16 and 32, both orientations, operands that are not
 16-byte aligned, beta*Y in place of the result, values that a bf16 split cannot hold.
 
 Bound.  One step of P products in precision u errs by at most (P + 2) u of the sum of the products' magnitudes
@@ -153,3 +154,21 @@ def test_split_pass_on_values_a_bf16_split_cannot_hold(lib, where, value):
         want, mag = xn @ fn, np.abs(xn) @ np.abs(fn)
     # 2^-149: the spacing of denormal results, once per product
     assert np.all((np.abs(z - want) <= 2.0 ** -24 * (P + 8) * mag + P * 2.0 ** -149)[ok])
+
+
+CHAIN = [
+    (1, [10] * 5, [10] * 5), (5, [12] * 4, [12] * 4), (300, [5] * 4, [5] * 4), (3, [14, 19, 34, 21], [15, 13, 23, 34]),
+    (1, [2] * 9, [2] * 9), (64, [3, 7], [9, 2]), (7, [32, 9, 5], [11, 31, 6]), (2, [1, 6, 1, 5], [3, 1, 2, 4]),
+    (1000, [11, 13], [13, 11]), (4, [3, 5, 16, 16], [3, 5, 16, 16]),
+]
+
+
+@pytest.mark.parametrize("mm,tx,tf,beta,shift", [("mkm", 0, 0, 0.0, 0), ("mkm", 1, 1, 1.0, 0), ("kmm", 0, 0, -0.5, 0),
+                                                 ("kmm", 1, 0, 0.0, 0), ("mkm", 0, 1, 1.0, 1)])
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("M,ps,qs", CHAIN, ids=lambda v: str(v).replace(" ", ""))
+def test_chain_launches(lib, M, ps, qs, dt, mm, tx, tf, beta, shift):
+    n0 = lib.fkbLaunchCount()
+    z, x, fs, y = call(mm, dt, M, ps, qs, tx, tf, beta, shift)
+    assert lib.fkbLaunchCount() - n0 < len(ps), "no two factors shared a launch"
+    check(z, x, fs, 2.0 if beta else 1.0, beta, y, 2.0 ** -24 if dt == "f32" else 2.0 ** -53)
