@@ -29,7 +29,7 @@
 // tiny throughout, below 2^-90, whose low parts would fall under the smallest bf16) are found while
 // splitting: such a row, or every row when the factor is concerned, is recomputed by its epilogue thread as
 // the plain FMA chain over p.
-#include <string.h>
+#include <stdlib.h>
 
 #include <cuda_bf16.h>
 
@@ -48,9 +48,10 @@ constexpr int kSplitRows = 128;
 constexpr int kSplitChunk = 16;                    // p per stage: a stage is 32 positions x 16 p of one converter warp
 constexpr int kSplitStageElems = 32 * kSplitChunk;
 constexpr int kSplitMaxStages = 5;
-constexpr int kSplitSmem = (227 - 22) * 1024;        // dynamic shared memory; the static part is below 22 KB
+constexpr int kSplitSmem = (227 - 3) * 1024;         // dynamic shared memory; the static part is below 3 KB
 constexpr unsigned kRowHuge = 1, kRowNormal = 2, kRowNonzero = 4;
-constexpr int kXposePitch = 20;                    // 16 columns and an odd number of 16-byte units per row
+constexpr int kXposePitch = 36;                    // 32 columns and an odd number of 16-byte units per row
+constexpr size_t kXposeBytes = kSplitEpiWarps * 32 * kXposePitch * sizeof(float);
 constexpr unsigned kHuge = 254u << 23;             // 2^127 as float bits
 constexpr unsigned kTiny = 37u << 23;              // 2^-90
 
@@ -58,7 +59,7 @@ struct SplitArgs {
   const float* X; float* Z; const float* Y; const float* F;
   long long fsP, fsQ;
   unsigned P, Q;
-  unsigned K, N;                                   // P and Q rounded up to 16
+  unsigned N;                                      // Q rounded up to 16
   unsigned stages;                                 // per converter warp, 1 .. kSplitMaxStages
   // position J = (i2*n1 + i1)*n0 + i0; element (J, p) of X at sum i*xs + p*xsP, (J, q) of Z and Y at sum i*zs + q*zsQ
   unsigned n0, n1;
@@ -71,14 +72,26 @@ struct SplitArgs {
   int outT, vecZ;                                  // the output is contiguous along q; 16-byte stores along it
 };
 
-// valid == false: nothing is read, the destination is zero-filled
+// Shared memory by its 32-bit address: two registers fewer per pointer, and none may be spilled here (with
+// all of the SM's memory taken as shared memory, a spilled register comes back from L2).
+// valid == false: nothing is read, the destination is zero-filled.
 template <int BYTES>
-__device__ __forceinline__ void cpAsyncFill(float* dst, const float* src, bool valid) {
+__device__ __forceinline__ void cpAsyncFill(unsigned dst, const float* src, bool valid) {
   const int n = valid ? BYTES : 0;
   if (BYTES == 16)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smemAddr(dst)), "l"(src), "r"(n) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
   else
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(smemAddr(dst)), "l"(src), "r"(n) : "memory");
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;\n" ::"r"(dst), "l"(src), "r"(n) : "memory");
+}
+__device__ __forceinline__ float ldShared(unsigned a) {
+  float v;
+  asm volatile("ld.shared.f32 %0, [%1];\n" : "=f"(v) : "r"(a) : "memory");
+  return v;
+}
+__device__ __forceinline__ float4 ldShared4(unsigned a) {
+  float4 v;
+  asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];\n" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(a) : "memory");
+  return v;
 }
 // all but the newest `n` groups of this thread are complete
 __device__ __forceinline__ void cpAsyncWaitUpTo(unsigned n) {
@@ -120,23 +133,25 @@ __device__ __forceinline__ void split2(float x0, float x1, unsigned& h, unsigned
 }
 
 // XT: the contracted index is contiguous in X (lanes load along p); otherwise lanes load along j.
-template <bool XT>
+// KS: steps of 16 along the contraction.
+template <bool XT, int KS>
 __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitArgs a) {
+  constexpr unsigned K = 16 * KS, ks = KS, half = K / 2;     // half: TMEM columns of one piece of A
+  constexpr unsigned slabs = (K + 63) / 64;
   extern __shared__ unsigned char smemRaw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
-  const unsigned slabs = (a.K + 63) / 64;
   const unsigned pieceBytes = slabs * a.N * 128u;            // one bf16 copy of the factor: [K/64][N rows q][64 k], 128-byte swizzle
   unsigned char* Fs = base;
-  float* ring = reinterpret_cast<float*>(base + 3 * pieceBytes);
+  float* xpose = reinterpret_cast<float*>(base + 3 * pieceBytes);                             // outT only
+  float* ring = xpose + (a.outT ? kXposeBytes / sizeof(float) : 0);
   __shared__ __align__(8) unsigned long long aFull[2], aEmpty[2], dFull[2], dEmpty[2];
   __shared__ unsigned tmemBaseSlot;
   __shared__ int abortFlag, factorSpecial;
   __shared__ unsigned colMax[128];
   __shared__ unsigned char rowState[4][2][kSplitRows];       // kRow* flags of a position, from its two converter warps
-  __shared__ __align__(16) float xpose[kSplitEpiWarps][32 * kXposePitch];
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const unsigned aCols = 3 * (a.K / 2);                      // TMEM columns of one A buffer: [h][m][l]
+  constexpr unsigned aCols = 3 * half;                     // TMEM columns of one A buffer: [h][m][l]
   const unsigned dCols = (a.N + 31) & ~31u;                  // one accumulator (read back 32 columns at a time)
   const unsigned nD = 2 * aCols + 2 * dCols <= 512 ? 2 : 1;  // accumulators; P, Q <= 128 leave room for one
 
@@ -166,12 +181,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     return max(__float_as_uint(v0) & 0x7FFFFFFFu, __float_as_uint(v1) & 0x7FFFFFFFu);
   };
   if (a.fsP != 1 || a.fsQ == 1) {
-    for (unsigned kp = warp; kp < a.K / 2; kp += kSplitThreads / 32)
+    for (unsigned kp = warp; kp < K / 2; kp += kSplitThreads / 32)
       for (unsigned q = lane; q < a.N; q += 32) atomicMax(&colMax[q], putFactor(kp, q));
   } else {
     for (unsigned q = warp; q < a.N; q += kSplitThreads / 32) {
       unsigned mx = 0;
-      for (unsigned kp = lane; kp < a.K / 2; kp += 32) mx = max(mx, putFactor(kp, q));
+      for (unsigned kp = lane; kp < K / 2; kp += 32) mx = max(mx, putFactor(kp, q));
       mx = __reduce_max_sync(0xffffffffu, mx);
       if (lane == 0) colMax[q] = mx;
     }
@@ -194,11 +209,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
 
   if (warp < kSplitEpiWarps) {
     // ---- epilogue ----------------------------------------------------------------------------
-    const unsigned quarter = (unsigned)warp & 3u, half = (unsigned)warp >> 2;
+    const unsigned quarter = (unsigned)warp & 3u, part = (unsigned)warp >> 2;
     const bool epi = a.epilogue != 0;
     const bool useY = epi && a.beta != 0.f && a.Y != nullptr;
     const bool allSpecial = factorSpecial != 0;
-    float* sc = xpose[warp];
+    float* sc = xpose + warp * 32 * kXposePitch;
     for (unsigned it = 0; it < myTiles; it++) {
       const unsigned d = nD == 2 ? (it & 1u) : 0u, use = nD == 2 ? (it >> 1) : it;
       const unsigned J = (first + it * step) * (unsigned)kSplitRows + quarter * 32u + (unsigned)lane;
@@ -214,7 +229,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
       const bool store = live && !special;
       const unsigned tcol = dCol + d * dCols + ((quarter * 32u) << 16);
 #pragma unroll 1
-      for (unsigned c0 = half * 32u; c0 < a.N || c0 < 64u; c0 += 64) {
+      for (unsigned c0 = part * 32u; c0 < a.N || c0 < 64u; c0 += 64) {
         unsigned r[32];
         if (c0 < a.N) {
           tmemLoad32(tcol + c0, r);
@@ -239,12 +254,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
           } else if (store) {
             const float* y = a.Y + zoff + (long long)c0 * a.zsQ;
 #pragma unroll
-            for (unsigned g = 0; g < 32; g += 8) {            // Y may be Z: read a batch ahead of its stores
-              float yv[8];
+            for (unsigned g = 0; g < 32; g += 4) {            // Y may be Z: read a batch ahead of its stores
+              float yv[4];
 #pragma unroll
-              for (unsigned i = 0; i < 8; i++) yv[i] = useY && c0 + g + i < a.Q ? y[(long long)(g + i) * a.zsQ] : 0.f;
+              for (unsigned i = 0; i < 4; i++) yv[i] = useY && c0 + g + i < a.Q ? y[(long long)(g + i) * a.zsQ] : 0.f;
 #pragma unroll
-              for (unsigned i = 0; i < 8; i++, z += a.zsQ) {
+              for (unsigned i = 0; i < 4; i++, z += a.zsQ) {
                 float v = a.alpha * __uint_as_float(r[g + i]);
                 if (useY) v = fmaf(a.beta, yv[i], v);
                 if (c0 + g + i < a.Q) *z = v;
@@ -252,48 +267,46 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
             }
           }
         } else {
-          // lanes hold positions, the output wants lanes along q: through the warp's scratch, 16 columns at a time
+          // Lanes hold positions, the output wants lanes along q: through the warp's scratch, 32 columns (a whole
+          // 128-byte line of every row) at a time.
           const unsigned stores = __ballot_sync(0xffffffffu, store);
 #pragma unroll
-          for (unsigned g = 0; g < 32; g += 16) {
+          for (unsigned i = 0; i < 32; i += 4)
+            *reinterpret_cast<uint4*>(sc + lane * kXposePitch + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+          __syncwarp();
+          if (a.vecZ) {
+            const unsigned q = c0 + 4 * ((unsigned)lane & 7u);           // Q % 4 == 0: whole vectors
 #pragma unroll
-            for (unsigned i = 0; i < 16; i += 4)
-              *reinterpret_cast<uint4*>(sc + lane * kXposePitch + i) = make_uint4(r[g + i], r[g + i + 1], r[g + i + 2], r[g + i + 3]);
-            __syncwarp();
-            if (a.vecZ) {
-              const unsigned q = c0 + g + 4 * ((unsigned)lane & 3u);     // Q % 4 == 0: whole vectors
-#pragma unroll
-              for (unsigned rr = (unsigned)lane >> 2, i = 0; i < 4; i++, rr += 8) {
-                const long long o = __shfl_sync(0xffffffffu, zoff, (int)rr) + q;
-                if (q < a.Q && (stores >> rr & 1u)) {
-                  float4 v = *reinterpret_cast<const float4*>(sc + rr * kXposePitch + 4 * (lane & 3));
-                  if (epi) {
-                    v.x = a.alpha * v.x; v.y = a.alpha * v.y; v.z = a.alpha * v.z; v.w = a.alpha * v.w;
-                    if (useY) {
-                      const float4 y = *reinterpret_cast<const float4*>(a.Y + o);
-                      v.x = fmaf(a.beta, y.x, v.x); v.y = fmaf(a.beta, y.y, v.y); v.z = fmaf(a.beta, y.z, v.z); v.w = fmaf(a.beta, y.w, v.w);
-                    }
+            for (unsigned rr = (unsigned)lane >> 3, i = 0; i < 8; i++, rr += 4) {
+              const long long o = __shfl_sync(0xffffffffu, zoff, (int)rr) + q;
+              if (q < a.Q && (stores >> rr & 1u)) {
+                float4 v = *reinterpret_cast<const float4*>(sc + rr * kXposePitch + 4 * (lane & 7));
+                if (epi) {
+                  v.x = a.alpha * v.x; v.y = a.alpha * v.y; v.z = a.alpha * v.z; v.w = a.alpha * v.w;
+                  if (useY) {
+                    const float4 y = *reinterpret_cast<const float4*>(a.Y + o);
+                    v.x = fmaf(a.beta, y.x, v.x); v.y = fmaf(a.beta, y.y, v.y); v.z = fmaf(a.beta, y.z, v.z); v.w = fmaf(a.beta, y.w, v.w);
                   }
-                  *reinterpret_cast<float4*>(a.Z + o) = v;
                 }
-              }
-            } else {
-              const unsigned q = c0 + g + ((unsigned)lane & 15u);
-#pragma unroll
-              for (unsigned rr = (unsigned)lane >> 4, i = 0; i < 16; i++, rr += 2) {
-                const long long o = __shfl_sync(0xffffffffu, zoff, (int)rr) + q;
-                if (q < a.Q && (stores >> rr & 1u)) {
-                  float v = sc[rr * kXposePitch + (lane & 15)];
-                  if (epi) { v = a.alpha * v; if (useY) v = fmaf(a.beta, a.Y[o], v); }
-                  a.Z[o] = v;
-                }
+                *reinterpret_cast<float4*>(a.Z + o) = v;
               }
             }
-            __syncwarp();
+          } else {
+            const unsigned q = c0 + (unsigned)lane;
+#pragma unroll 8
+            for (unsigned rr = 0; rr < 32; rr++) {
+              const long long o = __shfl_sync(0xffffffffu, zoff, (int)rr) + q;
+              if (q < a.Q && (stores >> rr & 1u)) {
+                float v = sc[rr * kXposePitch + lane];
+                if (epi) { v = a.alpha * v; if (useY) v = fmaf(a.beta, a.Y[o], v); }
+                a.Z[o] = v;
+              }
+            }
           }
+          __syncwarp();
         }
       }
-      if (special && half == 0) {
+      if (special && part == 0) {
         const float* x = a.X + (long long)i0 * a.xs0 + (long long)i1 * a.xs1 + (long long)i2 * a.xs2;
         for (unsigned q = 0; q < a.Q; q++) {
           float acc = 0.f;
@@ -308,20 +321,22 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     // ---- converters ----------------------------------------------------------------------------
     const unsigned cw = (unsigned)(warp - kSplitEpiWarps);
     const unsigned group = cw >> 3, sub = (cw >> 2) & 1u, quarter = cw & 3u;
-    float* const myRing = ring + (size_t)cw * a.stages * kSplitStageElems;
-    const unsigned ks = a.K / 16;                     // chunks; this warp takes sub, sub + 2, ...
+    constexpr unsigned stageBytes = kSplitStageElems * 4;
+    const unsigned myRing = smemAddr(ring) + cw * a.stages * stageBytes;
+    // this warp takes the chunks sub, sub + 2, ... of the ks
     const unsigned myGroupTiles = ks > sub && myTiles > group ? (myTiles - group + 1) / 2 : 0;
     // the loads run ahead of the conversion by the depth of the ring: tile ldTile (of this group), chunk ldC
     unsigned ldTile = 0, ldC = sub, ldMask = 0;
-    // Input offsets of what this lane fetches, once per tile: [0] the position along j (the first of four with
-    // 16-byte loads); with lanes along p, 16-byte loads: of the four rows lane / 4 + 8 i.  ldMask: which of them exist.
-    constexpr int NOFF = XT ? 4 : 1;
-    long long ldOff[NOFF];
+    // Input offsets of what this lane fetches, once per tile: ldOff of the position along j (the first of four with
+    // 16-byte loads), or, with lanes along p, of position `lane`; ldRow, 16-byte loads along p: of the rows
+    // lane / 4 + 8 i, in units of 16 bytes.  ldMask: which of them exist.
+    long long ldOff = 0;
+    unsigned ldRow[XT ? 4 : 1];
     auto offsetOf = [&](unsigned J) {
       const unsigned r0 = J / a.n0, i0 = J - r0 * a.n0, i2 = r0 / a.n1, i1 = r0 - i2 * a.n1;
       return (long long)i0 * a.xs0 + (long long)i1 * a.xs1 + (long long)i2 * a.xs2;
     };
-    auto load = [&](float* st) {
+    auto load = [&](unsigned st) {
       if (ldTile < myGroupTiles) {
         if (ldC == sub) {
           const unsigned J0 = (first + (2 * ldTile + group) * step) * (unsigned)kSplitRows + quarter * 32u;
@@ -329,18 +344,18 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
           if constexpr (!XT) {
             const unsigned j = a.vecX ? (unsigned)(lane & 7) * 4u : (unsigned)lane;   // n0 % 4 == 0 with 16-byte loads: whole vectors
             ldMask = j < rows ? 1u : 0u;
-            ldOff[0] = offsetOf(J0 + j);
+            ldOff = offsetOf(J0 + j);
           } else if (a.vecX) {
             const long long off = offsetOf(J0 + (unsigned)lane);
             ldMask = 0;
 #pragma unroll
             for (int i = 0; i < 4; i++) {
               const unsigned row = ((unsigned)lane >> 2) + 8u * i;
-              ldOff[i] = __shfl_sync(0xffffffffu, off, (int)row) + 4 * (lane & 3);
+              ldRow[i] = __shfl_sync(0xffffffffu, (unsigned)(off >> 2), (int)row) + ((unsigned)lane & 3u);
               if (row < rows) ldMask |= 1u << i;
             }
           } else {
-            ldOff[0] = offsetOf(J0 + (unsigned)lane);
+            ldOff = offsetOf(J0 + (unsigned)lane);
             ldMask = rows;
           }
         }
@@ -349,28 +364,28 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
         if constexpr (!XT) {
           if (a.vecX) {
             if (ldMask) {
-              const float* x = a.X + ldOff[0] + (long long)(p0 + ((unsigned)lane >> 3)) * a.xsP;
-              float* d = st + (lane >> 3) * 32 + (lane & 7) * 4;
+              const float* x = a.X + ldOff + (long long)(p0 + ((unsigned)lane >> 3)) * a.xsP;
+              const unsigned d = st + 16u * (unsigned)lane;
               if (whole) {
 #pragma unroll
-                for (int i = 0; i < 4; i++, x += 4 * a.xsP) cpAsyncFill<16>(d + i * 128, x, true);
+                for (int i = 0; i < 4; i++, x += 4 * a.xsP) cpAsyncFill<16>(d + i * 512, x, true);
               } else {
 #pragma unroll
                 for (unsigned i = 0; i < 4; i++, x += 4 * a.xsP) {
                   const bool ok = p0 + ((unsigned)lane >> 3) + 4 * i < a.P;
-                  cpAsyncFill<16>(d + i * 128, ok ? x : a.X, ok);
+                  cpAsyncFill<16>(d + i * 512, ok ? x : a.X, ok);
                 }
               }
             }
           } else if (ldMask) {
-            const float* x = a.X + ldOff[0] + (long long)p0 * a.xsP;
-            float* d = st + lane;
+            const float* x = a.X + ldOff + (long long)p0 * a.xsP;
+            const unsigned d = st + 4u * (unsigned)lane;
             if (whole) {
 #pragma unroll
-              for (int i = 0; i < kSplitChunk; i++, x += a.xsP) cpAsyncFill<4>(d + i * 32, x, true);
+              for (int i = 0; i < kSplitChunk; i++, x += a.xsP) cpAsyncFill<4>(d + i * 128, x, true);
             } else {
 #pragma unroll
-              for (unsigned i = 0; i < kSplitChunk; i++, x += a.xsP) cpAsyncFill<4>(d + i * 32, p0 + i < a.P ? x : a.X, p0 + i < a.P);
+              for (unsigned i = 0; i < kSplitChunk; i++, x += a.xsP) cpAsyncFill<4>(d + i * 128, p0 + i < a.P ? x : a.X, p0 + i < a.P);
             }
           }
         } else if (a.vecX) {
@@ -379,7 +394,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
           for (int i = 0; i < 4; i++) {
             const unsigned row = ((unsigned)lane >> 2) + 8u * i;
             if (ldMask >> i & 1u)
-              cpAsyncFill<16>(st + row * 16 + ((((unsigned)lane & 3u) ^ (row >> 1 & 3u)) << 2), okP ? a.X + ldOff[i] + p0 : a.X, okP);
+              cpAsyncFill<16>(st + row * 64 + ((((unsigned)lane & 3u) ^ (row >> 1 & 3u)) << 4), okP ? a.X + (4ll * ldRow[i] + p0) : a.X, okP);
           }
         } else {
           const unsigned pl = (unsigned)lane & 15u, p = p0 + pl;
@@ -388,8 +403,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
 #pragma unroll 8
           for (unsigned i = 0; i < 16; i++) {
             const unsigned row = ((unsigned)lane >> 4) + 2 * i;
-            const long long ro = __shfl_sync(0xffffffffu, ldOff[0], (int)row);
-            if (row < ldMask) cpAsyncFill<4>(st + row * 16 + ((((pl >> 2) ^ (row >> 1 & 3u)) << 2) | (pl & 3u)), okP ? xp + ro : a.X, okP);
+            const long long ro = __shfl_sync(0xffffffffu, ldOff, (int)row);
+            if (row < ldMask) cpAsyncFill<4>(st + row * 64 + ((((pl >> 2) ^ (row >> 1 & 3u)) << 4) | ((pl & 3u) << 2)), okP ? xp + ro : a.X, okP);
           }
         }
         ldC += 2;
@@ -397,10 +412,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
       }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
-    for (unsigned s = 0; s < a.stages; s++) load(myRing + s * kSplitStageElems);
+    for (unsigned s = 0; s < a.stages; s++) load(myRing + s * stageBytes);
     unsigned s = 0;
     const unsigned aBase = tmemBase + group * aCols + ((quarter * 32u) << 16);
-    const unsigned half = a.K / 2;
     for (unsigned li = 0; li < myGroupTiles; li++) {
       bool ok = !*abortP && waitBounded(&aEmpty[group], (li & 1u) ^ 1u, abortP);
       ok = __all_sync(0xffffffffu, ok);
@@ -412,15 +426,15 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
       for (unsigned c = sub; c < ks; c += 2) {
         cpAsyncWaitUpTo(a.stages - 1);
         __syncwarp();
-        float* st = myRing + s * kSplitStageElems;
+        const unsigned st = myRing + s * stageBytes;
         float x[16];
         if constexpr (!XT) {
 #pragma unroll
-          for (int i = 0; i < 16; i++) x[i] = st[i * 32 + lane];
+          for (int i = 0; i < 16; i++) x[i] = ldShared(st + i * 128 + 4 * lane);
         } else {
 #pragma unroll
           for (int i = 0; i < 4; i++) {
-            const float4 v = *reinterpret_cast<const float4*>(st + lane * 16 + ((i ^ (lane >> 1 & 3)) << 2));
+            const float4 v = ldShared4(st + lane * 64 + ((i ^ (lane >> 1 & 3)) << 4));
             x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
           }
         }
@@ -452,7 +466,6 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     // ---- MMA issue -------------------------------------------------------------------------------
     const unsigned elected = electOne();
     const unsigned idesc = splitInstrDesc(a.N);
-    const unsigned ks = a.K / 16, half = a.K / 2;
     const unsigned long long bDesc = smemDesc(smemAddr(Fs), 16u, 1024u, kSwz128);
     const unsigned pieceUnits = pieceBytes >> 4, slabUnits = a.N * 8u;   // descriptor addresses are in 16-byte units
     for (unsigned it = 0; it < myTiles; it++) {
@@ -463,25 +476,15 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
       if (!ok) break;
       fenceAfterSync();
       const unsigned tA = g * aCols, tD = 2 * aCols + d * dCols;         // the allocation is all of TMEM, it starts at 0
-      // one sweep over the contraction index: piece pa of X times piece pb of the factor
-      auto sweep = [&](unsigned pa, unsigned pb, bool fresh) {
-        unsigned ta = tA + pa * half;
-        unsigned long long bd = bDesc + pb * pieceUnits;
-        unsigned acc = fresh ? 0u : 1u;
-        for (unsigned k = 0; k < ks; k += 4, ta += 32u, bd += slabUnits) {
-          mmaBf16TmemA(elected, tD, ta, bd, idesc, acc);
-          acc = 1u;
-          if (k + 1 < ks) mmaBf16TmemA(elected, tD, ta + 8u, bd + 2u, idesc, 1u);
-          if (k + 2 < ks) mmaBf16TmemA(elected, tD, ta + 16u, bd + 4u, idesc, 1u);
-          if (k + 3 < ks) mmaBf16TmemA(elected, tD, ta + 24u, bd + 6u, idesc, 1u);
-        }
-      };
-      sweep(2, 0, true);
-      sweep(0, 2, false);
-      sweep(1, 1, false);
-      sweep(1, 0, false);
-      sweep(0, 1, false);
-      sweep(0, 0, false);
+      // six sweeps over the contraction index, the small terms first: piece pa of X times piece pb of the factor
+#pragma unroll
+      for (int t = 0; t < 6; t++) {
+        constexpr unsigned pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+        for (unsigned k = 0; k < ks; k++)
+          mmaBf16TmemA(elected, tD, tA + pa[t] * half + k * 8u, bDesc + pb[t] * pieceUnits + (k >> 2) * slabUnits + (k & 3u) * 2u, idesc,
+                       t > 0 || k > 0 ? 1u : 0u);
+      }
       if (elected) {
         mmaCommit(&aEmpty[g]);
         mmaCommit(&dFull[d]);
@@ -503,9 +506,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
 static unsigned long long gSplitLaunches = 0;
 static int gSplitOff = 0;                          // measurement hook fkbSetSplitOff
 
-template <bool XT>
+template <bool XT, int KS>
 static fastKronError launchSplitOne(const SplitArgs& a, const LaunchCtx& cx) {
-  auto kern = gemmSplitKernel<XT>;
+  auto kern = gemmSplitKernel<XT, KS>;
   static bool attrDev[kMaxDevices] = {false};
   bool& attr = attrDev[currentDeviceSlot()];
   if (!attr) {
@@ -523,6 +526,20 @@ static fastKronError launchSplitOne(const SplitArgs& a, const LaunchCtx& cx) {
   return cudaToFk(cudaGetLastError());
 }
 
+template <bool XT>
+static fastKronError launchSplitK(const SplitArgs& a, const LaunchCtx& cx) {
+  switch ((a.P + 15) / 16) {
+    case 2: return launchSplitOne<XT, 2>(a, cx);
+    case 3: return launchSplitOne<XT, 3>(a, cx);
+    case 4: return launchSplitOne<XT, 4>(a, cx);
+    case 5: return launchSplitOne<XT, 5>(a, cx);
+    case 6: return launchSplitOne<XT, 6>(a, cx);
+    case 7: return launchSplitOne<XT, 7>(a, cx);
+    case 8: return launchSplitOne<XT, 8>(a, cx);
+    default: return fastKronKernelNotFound;
+  }
+}
+
 }  // namespace tc
 
 // Passes this kernel takes; anything else returns fastKronKernelNotFound and runs on the FMA kernels.
@@ -536,7 +553,7 @@ fastKronError launchGemmSplit(const Pass& ps, const LaunchCtx& cx) {
   a.X = (const float*)cx.src; a.Z = (float*)cx.dst; a.Y = (const float*)cx.Y; a.F = (const float*)cx.F[0];
   a.fsP = cx.fsP; a.fsQ = cx.fsQ;
   a.P = ps.P[0]; a.Q = ps.Q[0];
-  a.K = (a.P + 15) / 16 * 16; a.N = (a.Q + 15) / 16 * 16;
+  a.N = (a.Q + 15) / 16 * 16;
   a.xsP = ps.xsG; a.zsQ = ps.zsG;
   a.alpha = (float)cx.alpha; a.beta = (float)cx.beta; a.epilogue = ps.epilogue ? 1 : 0;
   const bool xt = ps.xsG == 1;
@@ -550,15 +567,17 @@ fastKronError launchGemmSplit(const Pass& ps, const LaunchCtx& cx) {
   a.numTiles = (unsigned)((total + kSplitRows - 1) / kSplitRows);
   const bool al = ((uintptr_t)a.X & 15) == 0;
   auto m4 = [](int64_t v) { return v % 4 == 0; };
-  if (xt) a.vecX = al && a.P % 4 == 0 && (d[0].n == 1 || m4(a.xs0)) && (d[1].n == 1 || m4(a.xs1)) && (d[2].n == 1 || m4(a.xs2));
+  // (16-byte units of the input offset are 32-bit there)
+  const bool fits = d[0].n * (uint64_t)llabs(d[0].xs) + d[1].n * (uint64_t)llabs(d[1].xs) + d[2].n * (uint64_t)llabs(d[2].xs) < (1ull << 34);
+  if (xt) a.vecX = al && fits && a.P % 4 == 0 && (d[0].n == 1 || m4(a.xs0)) && (d[1].n == 1 || m4(a.xs1)) && (d[2].n == 1 || m4(a.xs2));
   else a.vecX = al && positionsVectorise(d, true, a.xsP, 4);
 
   a.vecZ = a.outT && a.Q % 4 == 0 && ((uintptr_t)a.Z & 15) == 0 && ((uintptr_t)a.Y & 15) == 0 && m4(a.zs0) && m4(a.zs1) && m4(a.zs2);
-  const size_t factor = 3 * (size_t)((a.K + 63) / 64) * a.N * 128;
+  const size_t factor = 3 * (size_t)((a.P + 63) / 64) * a.N * 128;
   const size_t stage = kSplitConvWarps * (size_t)kSplitStageElems * sizeof(float);    // one stage of every converter warp
-  const size_t n = (kSplitSmem - 1024 - factor) / stage;
+  const size_t n = (kSplitSmem - 1024 - factor - (a.outT ? kXposeBytes : 0)) / stage;
   a.stages = (unsigned)(n > kSplitMaxStages ? kSplitMaxStages : n);
-  return xt ? launchSplitOne<true>(a, cx) : launchSplitOne<false>(a, cx);
+  return xt ? launchSplitK<true>(a, cx) : launchSplitK<false>(a, cx);
 }
 
 int gemmSplitTimeouts() {

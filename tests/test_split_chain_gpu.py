@@ -82,7 +82,7 @@ def call(mm, dt, M, ps, qs, tx, tf, beta, shift, seed=0):
 SPLIT = [
     # M, ps, qs
     (128, [33, 17], [32, 61]), (40, [64, 64], [64, 64]), (9, [127, 128], [128, 127]), (33, [128, 40], [96, 128]),
-    (17, [65, 80], [113, 49]), (20, [48, 112], [112, 48]), (1, [64, 33, 34], [33, 64, 36]), (300, [128, 128], [128, 128]),
+    (17, [65, 80], [113, 49]), (24, [48, 112], [112, 48]), (1, [64, 33, 34], [33, 64, 36]), (300, [128, 128], [128, 128]),
 ]
 
 
