@@ -37,11 +37,13 @@ inline bool gemmAnyEligible(uint32_t P, uint32_t Q) {
 }
 
 // The split tensor-core kernel (kernel_gemm_split.cu), fp32: factors up to 128 on either side; `total` is the
-// number of positions (rows of the contraction).  Smaller factors leave the FMA kernels bound by memory already
-// (256 rows, 24x24 three times: 58 us, against 78 us with the split kernel's fixed work per position), and below 1024
-// positions the eight tiles of 128 leave most of the chip idle.
+// number of positions (rows of the contraction).  Measured on B200, FMA kernels -> this one, 25 million elements, pass
+// with p contiguous / with j contiguous: 36x36 182/158 -> 83/68 us, 64x64 85/84 -> 59/48, 100x100 229/207 -> 67/62; 48 -> 24 columns 51/27
+// -> 48/25, about even, and 64 -> 17 loses (55/21 -> 67/17: the fixed work per tile is spread over few outputs).  Below 24x24 the FMA
+// kernels are bound by memory themselves (24x24 three times, 256 rows: 58 us, 78 us here).  From 1024 positions (eight tiles)
+// on the launches take the same time (64x64: 12.4 and 13.7 us); fewer have never been faster here.
 inline bool gemmSplitEligible(uint32_t P, uint32_t Q, uint64_t total) {
-  return P >= 17 && Q >= 17 && P <= 128 && Q <= 128 && P * Q >= 1024 && total >= 1024 && total < (1ull << 31);
+  return P >= 17 && Q >= 20 && P <= 128 && Q <= 128 && P * Q >= 1024 && total >= 1024 && total < (1ull << 31);
 }
 
 }  // namespace fkb

@@ -25,6 +25,12 @@
 //         registers, where the instruction wants them) and one elected lane issues
 // Every wait on a barrier is bounded; one that gives up raises the abort flag that ends all roles.
 //
+// Bound by HBM traffic and, where P is small, by the fixed work of a tile.  Measured on B200, 268 MB in and out (81 us at the copy
+// rate), 64x64: 97 us a pass with j contiguous (FMA kernel 187), 127 us with p contiguous (cold X; 59 against 85 us at
+// 100 MB); 128x128 and 134 MB (40 us): 64 / 74 us (FMA 320).  The contraction length is a template parameter because the MMAs are issued by
+// one lane: with run-time descriptors a 128x64x16 MMA took 126-152 clocks, with immediate ones the passes no longer
+// notice twice the MMAs.
+//
 // Operands a bf16 split cannot hold (infinities, NaN, magnitudes from 2^127; rows or factor columns that are
 // tiny throughout, below 2^-90, whose low parts would fall under the smallest bf16) are found while
 // splitting: such a row, or every row when the factor is concerned, is recomputed by its epilogue thread as
@@ -213,6 +219,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     const bool epi = a.epilogue != 0;
     const bool useY = epi && a.beta != 0.f && a.Y != nullptr;
     const bool allSpecial = factorSpecial != 0;
+    const bool linear = a.n0 == a.total;
     float* sc = xpose + warp * 32 * kXposePitch;
     for (unsigned it = 0; it < myTiles; it++) {
       const unsigned d = nD == 2 ? (it & 1u) : 0u, use = nD == 2 ? (it >> 1) : it;
@@ -274,32 +281,53 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
           for (unsigned i = 0; i < 32; i += 4)
             *reinterpret_cast<uint4*>(sc + lane * kXposePitch + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
           __syncwarp();
+          // offset of row rr of this warp's 32, also on lanes whose own position lies beyond the last
+          auto rowOff = [&](unsigned rr) -> long long {
+            if (linear) return (long long)(J - (unsigned)lane + rr) * a.zs0;
+            return __shfl_sync(0xffffffffu, zoff, (int)rr);
+          };
+          // (reads of a batch of rows ahead of their stores: a store may alias the scratch as far as the compiler knows)
           if (a.vecZ) {
             const unsigned q = c0 + 4 * ((unsigned)lane & 7u);           // Q % 4 == 0: whole vectors
+#pragma unroll 1
+            for (unsigned b = 0; b < 32; b += 8) {
+              float4 v[2];
+              long long o[2];
 #pragma unroll
-            for (unsigned rr = (unsigned)lane >> 3, i = 0; i < 8; i++, rr += 4) {
-              const long long o = __shfl_sync(0xffffffffu, zoff, (int)rr) + q;
-              if (q < a.Q && (stores >> rr & 1u)) {
-                float4 v = *reinterpret_cast<const float4*>(sc + rr * kXposePitch + 4 * (lane & 7));
+              for (unsigned i = 0; i < 2; i++) {
+                const unsigned rr = b + 4 * i + ((unsigned)lane >> 3);
+                v[i] = *reinterpret_cast<const float4*>(sc + rr * kXposePitch + 4 * (lane & 7));
+                o[i] = rowOff(rr) + q;
+              }
+#pragma unroll
+              for (unsigned i = 0; i < 2; i++) {
+                const unsigned rr = b + 4 * i + ((unsigned)lane >> 3);
+                if (q >= a.Q || !(stores >> rr & 1u)) continue;
                 if (epi) {
-                  v.x = a.alpha * v.x; v.y = a.alpha * v.y; v.z = a.alpha * v.z; v.w = a.alpha * v.w;
+                  v[i].x = a.alpha * v[i].x; v[i].y = a.alpha * v[i].y; v[i].z = a.alpha * v[i].z; v[i].w = a.alpha * v[i].w;
                   if (useY) {
-                    const float4 y = *reinterpret_cast<const float4*>(a.Y + o);
-                    v.x = fmaf(a.beta, y.x, v.x); v.y = fmaf(a.beta, y.y, v.y); v.z = fmaf(a.beta, y.z, v.z); v.w = fmaf(a.beta, y.w, v.w);
+                    const float4 y = *reinterpret_cast<const float4*>(a.Y + o[i]);
+                    v[i].x = fmaf(a.beta, y.x, v[i].x); v[i].y = fmaf(a.beta, y.y, v[i].y);
+                    v[i].z = fmaf(a.beta, y.z, v[i].z); v[i].w = fmaf(a.beta, y.w, v[i].w);
                   }
                 }
-                *reinterpret_cast<float4*>(a.Z + o) = v;
+                *reinterpret_cast<float4*>(a.Z + o[i]) = v[i];
               }
             }
           } else {
             const unsigned q = c0 + (unsigned)lane;
-#pragma unroll 8
-            for (unsigned rr = 0; rr < 32; rr++) {
-              const long long o = __shfl_sync(0xffffffffu, zoff, (int)rr) + q;
-              if (q < a.Q && (stores >> rr & 1u)) {
-                float v = sc[rr * kXposePitch + lane];
-                if (epi) { v = a.alpha * v; if (useY) v = fmaf(a.beta, a.Y[o], v); }
-                a.Z[o] = v;
+#pragma unroll 2
+            for (unsigned b = 0; b < 32; b += 4) {
+              float v[4];
+#pragma unroll
+              for (unsigned i = 0; i < 4; i++) v[i] = sc[(b + i) * kXposePitch + lane];
+#pragma unroll
+              for (unsigned i = 0; i < 4; i++) {
+                const long long o = rowOff(b + i) + q;
+                if (q < a.Q && (stores >> (b + i) & 1u)) {
+                  if (epi) { v[i] = a.alpha * v[i]; if (useY) v[i] = fmaf(a.beta, a.Y[o], v[i]); }
+                  a.Z[o] = v[i];
+                }
               }
             }
           }
@@ -572,7 +600,8 @@ fastKronError launchGemmSplit(const Pass& ps, const LaunchCtx& cx) {
   if (xt) a.vecX = al && fits && a.P % 4 == 0 && (d[0].n == 1 || m4(a.xs0)) && (d[1].n == 1 || m4(a.xs1)) && (d[2].n == 1 || m4(a.xs2));
   else a.vecX = al && positionsVectorise(d, true, a.xsP, 4);
 
-  a.vecZ = a.outT && a.Q % 4 == 0 && ((uintptr_t)a.Z & 15) == 0 && ((uintptr_t)a.Y & 15) == 0 && m4(a.zs0) && m4(a.zs1) && m4(a.zs2);
+  a.vecZ = a.outT && a.Q % 4 == 0 && ((uintptr_t)a.Z & 15) == 0 && ((uintptr_t)a.Y & 15) == 0 && (d[0].n == 1 || m4(a.zs0)) &&
+           (d[1].n == 1 || m4(a.zs1)) && (d[2].n == 1 || m4(a.zs2));
   const size_t factor = 3 * (size_t)((a.P + 63) / 64) * a.N * 128;
   const size_t stage = kSplitConvWarps * (size_t)kSplitStageElems * sizeof(float);    // one stage of every converter warp
   const size_t n = (kSplitSmem - 1024 - factor - (a.outT ? kXposeBytes : 0)) / stage;
