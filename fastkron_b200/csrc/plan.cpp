@@ -22,6 +22,8 @@
 #include "tile_db.h"
 #include "chain_table.h"
 
+#include <algorithm>
+#include <cmath>
 #include <sstream>
 #include <stdlib.h>
 
@@ -277,20 +279,31 @@ static Pass groupPass(const Problem& pr, int f0, int f1) {
   return ps;
 }
 
-// Estimated device time (us) of factors f0 .. f1 in one launch; negative when they do not fit.
+// Estimated device time (us) of factors f0 .. f1 in one launch; negative when they do not fit.  Rates from B200:
+// the single-factor kernel reaches 3.0 TB/s and, on full tiles, 13e12 (fp32) or 3.9e12 (fp64) multiply-adds per second,
+// less by what a factor leaves of its tile (64, 32 or 16 wide, chunks of 32 or 16); a chain 5.0 TB/s and 7.5e12 or 3.2e12, in
+// whole waves of CTAs.  (Two of 31x31x31 fp64 in one launch: 66 us against 23 + 23, which the bytes alone do not say;
+// three of 12x12 fp32: 100 us against 87 + 61 + 55.)
 static double groupCost(const Problem& pr, int f0, int f1) {
   const Pass ps = groupPass(pr, f0, f1);
+  const bool f32 = pr.dt == DType::F32;
   const double es = (double)dtypeSize(pr.dt), pos = (double)ps.M * ps.A * ps.B;
   const double bytes = pos * ((double)ps.Pg() + (double)ps.Qg()) * es;
   if (pos >= 2147483648.0) return -1;
-  if (f0 == f1) return 3 + bytes / 3.0e6;            // the single-factor kernels
+  double macs = 0, cols = (double)ps.Pg();
+  for (int k = ps.nf - 1; k >= 0; k--) { cols = cols / ps.P[k] * ps.Q[k]; macs += pos * cols * ps.P[k]; }
+  if (f0 == f1) {
+    const unsigned P = ps.P[0], Q = ps.Q[0], tq = Q <= 16 ? 16 : Q <= 32 ? 32 : (Q + 63) / 64 * 64, pc = Q <= 32 ? 16 : 32;
+    const double fill = (double)Q / tq * P / ((P + pc - 1) / pc * pc);
+    return 4 + std::max(bytes / 3.0e6, macs / ((f32 ? 13e6 : 3.9e6) * fill));
+  }
   ChainShape s;
   if (!chainShape(pr.dt, ps.nf, ps.P, ps.Q, ps.xsG == 1 || ps.zsG == 1, (uint64_t)pos, &s)) return -1;
   // short runs of a strided side cost sectors
   double runs = 1;
   if (ps.xsG != 1 || ps.zsG != 1) { const double run = s.W * es; runs = run >= 64 ? 1 : run >= 32 ? 1.3 : 1.8; }
-  if (s.smem > kChainSmem3) runs *= 1.15;
-  return 3 + bytes / 5.0e6 * runs;
+  const double waves = std::ceil(pos / s.W) / (148.0 * (s.smem > kChainSmem3 ? 2 : 3));
+  return 4 + std::max(bytes / 5.0e6 * runs, macs / (f32 ? 7.5e6 : 3.2e6)) * (waves > 1 ? std::ceil(waves) / waves : 1);
 }
 
 void fuseLaunches(const Problem& pr, const PlanOptions& opt, Plan* plan) {
