@@ -7,6 +7,8 @@ sm_100a) reached through the C ABI of ``include/fastkron.h``; torch is used only
 for device memory and streams.  There is no CPU path.
 """
 import ctypes
+import functools
+import math
 from typing import List, Optional
 
 from . import lib as _lib
@@ -171,18 +173,42 @@ def gekmm_sizes(M, ps, qs):
     return _handle().sizes(M, ps, qs)
 
 
+# What a call needs besides its operands, per factor shapes: the C arrays (the library only reads them), the
+# sides of the product and the widest matrix of any single-factor step per row of X (gekmmSizes).
+@functools.lru_cache(maxsize=256)
+def _shape(ps, qs):
+    k, l = math.prod(ps), math.prod(qs)
+    cols = k
+    widest = max(k, l) if len(ps) == 1 else 0
+    for p, q in zip(reversed(ps), reversed(qs)):
+        cols = cols // p * q if p else 0
+        widest = max(widest, cols)
+    return k, l, widest, _lib.u32arr(ps), _lib.u32arr(qs)
+
+
+# The four front-end entry points with argument types of their own (independent of the library handle's
+# functions, whose callers pass ctypes objects).
+@functools.lru_cache(maxsize=None)
+def _entry(lib, mm, dch):
+    i, u, vp = ctypes.c_int, ctypes.c_uint32, ctypes.c_void_p
+    sc = ctypes.c_float if dch == "s" else ctypes.c_double
+    head = (vp, i, u, u, vp, vp, vp, i, vp, i) if mm == "mkm" else (vp, i, u, vp, vp, u, vp, i, vp, i)
+    return ctypes.CFUNCTYPE(i, *head, vp, sc, sc, vp, vp, vp)((dch + ("gemkm" if mm == "mkm" else "gekmm"), lib))
+
+
 def _run(mm, x, fs, alpha, beta, y):
     torch = _torch()
     if not x.is_cuda:
         raise ValueError("fastkron_b200 computes on CUDA tensors only")
-    if x.dtype not in (torch.float32, torch.float64):
+    dtype, device = x.dtype, x.device
+    if dtype not in (torch.float32, torch.float64):
         raise TypeError("only float32 and float64 are supported")
     h = _handle()
-    dch = "s" if x.dtype == torch.float32 else "d"
+    dch, es = ("s", 4) if dtype == torch.float32 else ("d", 8)
     xs, trx = _as_op(x)
     fstore, trfs = [], []
     for f in fs:
-        if f.dtype != x.dtype or f.device != x.device:
+        if f.dtype != dtype or f.device != device:
             raise TypeError("factors must match x in dtype and device")
         s, t = _as_op(f)
         fstore.append(s)
@@ -192,24 +218,18 @@ def _run(mm, x, fs, alpha, beta, y):
     for i, f in enumerate(fs):
         if trfs[i] != trf:
             fstore[i] = (f.t().contiguous() if trf else f.contiguous())
+    shapes = [tuple(f.shape) for f in fs]
     if mm == "mkm":
         M, K = x.shape
-        ps = [f.shape[0] for f in fs]
-        qs = [f.shape[1] for f in fs]
+        ps, qs = tuple(s[0] for s in shapes), tuple(s[1] for s in shapes)
     else:
         K, M = x.shape
-        qs = [f.shape[0] for f in fs]
-        ps = [f.shape[1] for f in fs]
-    kk = 1
-    for p in ps:
-        kk *= p
+        qs, ps = tuple(s[0] for s in shapes), tuple(s[1] for s in shapes)
+    kk, L, cols, P, Q = _shape(ps, qs)
     if kk != K:
         raise ValueError("product of factor sizes (%d) does not match x (%d)" % (kk, K))
-    L = 1
-    for q in qs:
-        L *= q
     zshape = (M, L) if mm == "mkm" else (L, M)
-    z = torch.empty(zshape, dtype=x.dtype, device=x.device)
+    z = torch.empty(zshape, dtype=dtype, device=device)
     yptr = 0
     if y is not None and beta != 0:
         if tuple(y.shape) != zshape:
@@ -218,12 +238,23 @@ def _run(mm, x, fs, alpha, beta, y):
         yptr = y.data_ptr()
     elif beta != 0:
         raise ValueError("beta != 0 needs y")
-    _, te = h.sizes(M, ps, qs)
-    t1 = torch.empty(te, dtype=x.dtype, device=x.device)
-    t2 = torch.empty(te, dtype=x.dtype, device=x.device)
-    h.raw_gemm(mm, dch, M, ps, qs, xs.data_ptr(), _lib.OP_T if trx else _lib.OP_N,
-               [f.data_ptr() for f in fstore], _lib.OP_T if trf else _lib.OP_N,
-               z.data_ptr(), float(alpha), float(beta), yptr, t1.data_ptr(), t2.data_ptr())
+    n = len(shapes)
+    if n == 0 or n > 64:
+        h.sizes(M, ps, qs)          # raises what the library says to such a problem
+    # small temporaries from one allocation, the second on a 16-byte boundary; large ones each from its own
+    half = -(-M * cols * es // 16) * 16
+    temps = [torch.empty(2 * half, dtype=torch.uint8, device=device)] if half <= 1 << 20 else \
+            [torch.empty(half, dtype=torch.uint8, device=device) for _ in range(2)]
+    t1 = temps[0].data_ptr()
+    t2 = t1 + half if len(temps) == 1 else temps[1].data_ptr()
+    F = (ctypes.c_void_p * n)(*[f.data_ptr() for f in fstore])
+    opx, opf = _lib.OP_T if trx else _lib.OP_N, _lib.OP_T if trf else _lib.OP_N
+    fn = _entry(h.lib, mm, dch)
+    if mm == "mkm":
+        rc = fn(h.h, _lib.BACKEND_CUDA, M, n, P, Q, xs.data_ptr(), opx, F, opf, z.data_ptr(), float(alpha), float(beta), yptr, t1, t2)
+    else:
+        rc = fn(h.h, _lib.BACKEND_CUDA, n, Q, P, M, F, opf, xs.data_ptr(), opx, z.data_ptr(), float(alpha), float(beta), yptr, t1, t2)
+    _lib.check(rc)
     return z
 
 

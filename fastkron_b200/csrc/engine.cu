@@ -84,6 +84,17 @@ static std::string planKey(const Problem& pr, const PlanOptions& o) {
   return os.str();
 }
 
+// The same distinctions as bytes: what the plan cache is looked up by on every call (building the text took
+// longer than the lookup).
+static std::string planCacheKey(const Problem& pr, const PlanOptions& o) {
+  const uint32_t head[] = {(uint32_t)pr.mm, (uint32_t)pr.dt, pr.M, pr.N, (uint32_t)pr.opX, (uint32_t)pr.opF, pr.forward, pr.batch > 1,
+                           o.fusion, o.haveT2, o.forceGeneric, (uint32_t)o.align};
+  std::string k(reinterpret_cast<const char*>(head), sizeof(head));
+  k.append(reinterpret_cast<const char*>(pr.P), pr.N * sizeof(pr.P[0]));
+  k.append(reinterpret_cast<const char*>(pr.Q), pr.N * sizeof(pr.Q[0]));
+  return k;
+}
+
 // 0 = silent, 1 = INFO, 2 = DEBUG; read once from FASTKRON_LOG.
 static int logLevel() {
   static const int lv = [] {
@@ -162,7 +173,7 @@ fastKronError Engine::run(Problem pr, const CallOperands& ops) {
     }
   }
 
-  const std::string key = planKey(pr, po);
+  const std::string key = planCacheKey(pr, po);
   auto it = planCache_.find(key);
   if (it == planCache_.end()) {
     Plan plan;
@@ -197,7 +208,7 @@ fastKronError Engine::run(Problem pr, const CallOperands& ops) {
     }
     // FASTKRON_LOG=INFO (or DEBUG): one block per newly planned problem, as the reference prints
     // its chosen kernel series (src/env/env.cpp:57-65, src/handle/handle.cpp:160-170).
-    if (logLevel() >= 1) fprintf(stderr, "[FastKron] plan %s\n%s", key.c_str(), plan.describe().c_str());
+    if (logLevel() >= 1) fprintf(stderr, "[FastKron] plan %s\n%s", planKey(pr, po).c_str(), plan.describe().c_str());
     it = planCache_.emplace(key, std::move(plan)).first;
   }
   const Plan& plan = it->second;
