@@ -31,8 +31,9 @@
 // one lane: with run-time descriptors a 128x64x16 MMA took 126-152 clocks, with immediate ones the passes no longer
 // notice twice the MMAs.
 //
-// Operands a bf16 split cannot hold (infinities, NaN, magnitudes from 2^127; rows or factor columns that are
-// tiny throughout, below 2^-90, whose low parts would fall under the smallest bf16) are found while
+// Operands a bf16 split cannot hold (infinities, NaN, magnitudes from 2^127 or whose sums could overflow; rows or
+// factor columns that are tiny throughout, below 2^-90 or 2^-100 together, whose low parts would fall under the
+// smallest normal numbers) are found while
 // splitting: such a row, or every row when the factor is concerned, is recomputed by its epilogue thread as
 // the plain FMA chain over p.
 #include <stdlib.h>
@@ -153,6 +154,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   __shared__ __align__(8) unsigned long long aFull[2], aEmpty[2], dFull[2], dEmpty[2];
   __shared__ unsigned tmemBaseSlot;
   __shared__ int abortFlag, factorSpecial;
+  __shared__ unsigned factorMax, factorMin;                 // float bits: largest and smallest nonzero column maximum
   __shared__ unsigned colMax[128];
   __shared__ unsigned char rowState[4][2][kSplitRows];       // kRow* flags of a position, from its two converter warps
 
@@ -164,6 +166,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   if (tid == 0) {
     for (int i = 0; i < 2; i++) { mbarInit(&aFull[i], kSplitConvWarps / 2); mbarInit(&aEmpty[i], 1); mbarInit(&dFull[i], 1); mbarInit(&dEmpty[i], kSplitEpiWarps); }
     abortFlag = 0; factorSpecial = 0;
+    factorMax = 0; factorMin = kHuge;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == kSplitMmaWarp) {
@@ -204,6 +207,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   if (tid < 128) {
     const unsigned c = colMax[tid];
     if (c >= kHuge || (c != 0 && c < kTiny)) factorSpecial = 1;
+    atomicMax(&factorMax, c);
+    if (c != 0) atomicMin(&factorMin, c);
   }
   __syncthreads();
   const unsigned tmemBase = *(volatile unsigned*)&tmemBaseSlot;
@@ -482,8 +487,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
         tmemStore8(col + 2 * half, l);
       }
       const unsigned bits = __float_as_uint(__bfloat162float(__hmax_nan(__low2bfloat16(mx), __high2bfloat16(mx))));
+      // magnitudes at which a sum of 128 products may pass 2^126 (terms of a split could become infinities of
+      // opposite signs) or the low terms of a column fall below the normal numbers
+      const unsigned huge = min(kHuge, __float_as_uint(0x1p119f / __uint_as_float(factorMax)));
+      const unsigned tiny = max(kTiny, __float_as_uint(0x1p-100f / __uint_as_float(factorMin)));
       rowState[(2 * li + group) & 3][sub][quarter * 32 + lane] =
-          (unsigned char)((bits >= kHuge ? kRowHuge : 0u) | (bits >= kTiny ? kRowNormal : 0u) | ((any << 1) != 0 ? kRowNonzero : 0u));
+          (unsigned char)((bits >= huge ? kRowHuge : 0u) | (bits >= tiny ? kRowNormal : 0u) | ((any << 1) != 0 ? kRowNonzero : 0u));
       tmemStoreWait();
       fenceBeforeSync();
       __syncwarp();

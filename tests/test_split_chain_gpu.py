@@ -156,6 +156,28 @@ def test_split_pass_on_values_a_bf16_split_cannot_hold(lib, where, value):
     assert np.all((np.abs(z - want) <= 2.0 ** -24 * (P + 8) * mag + P * 2.0 ** -149)[ok])
 
 
+@pytest.mark.parametrize("xs,fs", [(1e38, 1e10), (1e30, 1e9), (1e20, 1e20), (3e37, 1.0), (1e-25, 1e-10), (1e-20, 1e-20), (1e15, 1e-26)])
+def test_split_pass_at_the_ends_of_the_range(lib, xs, fs):
+    """Products that overflow give the infinities of the FMA chain and no NaN; small ones keep their precision."""
+    import torch
+    import fastkron_b200
+    torch.manual_seed(2)
+    M, P, Q = 1500, 64, 48
+    x, f = (torch.rand(M, P, device="cuda") + 0.5), (torch.rand(P, Q, device="cuda") + 0.5) * fs
+    x[1::7] *= xs
+    n0 = lib.fkbGemmSplitLaunches()
+    z = fastkron_b200.gemkm(x, [f]).cpu().numpy().astype(np.float64)
+    assert lib.fkbGemmSplitLaunches() == n0 + 1
+    lib.fkbSetSplitOff(1)
+    w = fastkron_b200.gemkm(x, [f]).cpu().numpy().astype(np.float64)
+    lib.fkbSetSplitOff(0)
+    assert not np.isnan(z).any() and np.array_equal(np.isinf(z), np.isinf(w))
+    xn, fn = x.cpu().numpy().astype(np.float64), f.cpu().numpy().astype(np.float64)
+    ok = np.isfinite(w)
+    err = np.abs(np.where(ok, z, 0) - np.where(ok, xn @ fn, 0))
+    assert np.all(err <= 2.0 ** -24 * (P + 8) * (xn @ fn) + P * 2.0 ** -149)
+
+
 CHAIN = [
     (1, [10] * 5, [10] * 5), (5, [12] * 4, [12] * 4), (300, [5] * 4, [5] * 4), (3, [14, 19, 34, 21], [15, 13, 23, 34]),
     (1, [2] * 9, [2] * 9), (64, [3, 7], [9, 2]), (7, [32, 9, 5], [11, 31, 6]), (2, [1, 6, 1, 5], [3, 1, 2, 4]),
