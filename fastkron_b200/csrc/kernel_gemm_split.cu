@@ -154,6 +154,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   __shared__ __align__(8) unsigned long long aFull[2], aEmpty[2], dFull[2], dEmpty[2];
   __shared__ unsigned tmemBaseSlot;
   __shared__ int abortFlag, factorSpecial;
+  __shared__ unsigned rowHuge, rowTiny;
   __shared__ unsigned factorMax, factorMin;                 // float bits: largest and smallest nonzero column maximum
   __shared__ unsigned colMax[128];
   __shared__ unsigned char rowState[4][2][kSplitRows];       // kRow* flags of a position, from its two converter warps
@@ -209,6 +210,13 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     if (c >= kHuge || (c != 0 && c < kTiny)) factorSpecial = 1;
     atomicMax(&factorMax, c);
     if (c != 0) atomicMin(&factorMin, c);
+  }
+  __syncthreads();
+  if (tid == 0) {
+    // row magnitudes at which a sum of 128 products may pass 2^126 (terms of a split could become infinities of
+    // opposite signs) or the low terms of a column fall below the normal numbers
+    rowHuge = min(kHuge, __float_as_uint(0x1p119f / __uint_as_float(factorMax)));
+    rowTiny = max(kTiny, __float_as_uint(0x1p-100f / __uint_as_float(factorMin)));
   }
   __syncthreads();
   const unsigned tmemBase = *(volatile unsigned*)&tmemBaseSlot;
@@ -487,12 +495,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
         tmemStore8(col + 2 * half, l);
       }
       const unsigned bits = __float_as_uint(__bfloat162float(__hmax_nan(__low2bfloat16(mx), __high2bfloat16(mx))));
-      // magnitudes at which a sum of 128 products may pass 2^126 (terms of a split could become infinities of
-      // opposite signs) or the low terms of a column fall below the normal numbers
-      const unsigned huge = min(kHuge, __float_as_uint(0x1p119f / __uint_as_float(factorMax)));
-      const unsigned tiny = max(kTiny, __float_as_uint(0x1p-100f / __uint_as_float(factorMin)));
       rowState[(2 * li + group) & 3][sub][quarter * 32 + lane] =
-          (unsigned char)((bits >= huge ? kRowHuge : 0u) | (bits >= tiny ? kRowNormal : 0u) | ((any << 1) != 0 ? kRowNonzero : 0u));
+          (unsigned char)((bits >= rowHuge ? kRowHuge : 0u) | (bits >= rowTiny ? kRowNormal : 0u) | ((any << 1) != 0 ? kRowNonzero : 0u));
       tmemStoreWait();
       fenceBeforeSync();
       __syncwarp();
