@@ -498,6 +498,10 @@ def dominant_roofline(c, passes, flops, peaks, peak_src, fma_probe, fma_props):
                     "unit": "TFLOP/s", "frac": fp_ach / fp_peak,
                     "peak_source": "larger of the FMA-chain probe of this run (%.1f) and SMs x lanes x 2 x max SM clock "
                                    "from the device properties (%.1f)" % (fma_probe or 0.0, fma_props or 0.0)}, **common)
+    # large fp32 factors run on the tensor cores (exact bf16 splits): the FMA rate bounds nothing there
+    from fastkron_b200 import lib as fk
+    if kind == "gemm" and c["dt"] == "f32" and fk.get().fkbGemmSplitLaunches() > 0:
+        return dict(roof_hbm, other=roof_fp)
     return dict(roof_fp, other=roof_hbm) if roof_fp["frac"] > roof_hbm["frac"] else dict(roof_hbm, other=roof_fp)
 
 
