@@ -656,7 +656,7 @@ def run_single(args):
         "gpu_launches": r["launches"], "passes": passes, "clocks": clocks, "roofline": roof, "e2e": e2e,
         "cpu_baseline": cpu, "parity_rows_max_rel_err": parity,
         "fma_peak_tflops": {"probe": fma_probe, "device_props": fma_props}, "configs": extra, "any_shape_kernel": any_table, "tf32_optin": tf32, "tf32x3_optin": tf32x3,
-        "gemm_timeouts": int(fk.get().fkbGemmTmaTimeouts()),
+        "gemm_timeouts": int(fk.get().fkbGemmTmaTimeouts()) | int(fk.get().fkbGemmSplitTimeouts()),
     }
     print(json.dumps(out))
 

@@ -58,6 +58,17 @@ def test_option_bits_keep_reference_values_and_tf32_is_an_extra_bit(tmp_path):
     assert hasattr(Lh, "fkbGemmTcTimeouts") and hasattr(Lh, "fkbGemmTmaTimeouts")
 
 
+def test_device_status_asks_every_kernel_with_bounded_waits(L):
+    """Each kernel family whose waits can give up exports fkb<family>Timeouts(); fkbDeviceStatus() may only report
+    success when none of them has (a wait that gives up leaves tiles unwritten)."""
+    out = subprocess.run(["nm", "-D", "--defined-only", L._name], capture_output=True, text=True, check=True).stdout
+    families = set(re.findall(r"\bfkb\w+Timeouts\b", out))
+    assert len(families) >= 4, families
+    src = open(os.path.join(ROOT, "fastkron_b200", "csrc", "api.cu")).read()
+    body = re.search(r"fastKronError fkbDeviceStatus\(\) \{(.*?)\n\}", src, re.S).group(1)
+    assert families == set(re.findall(r"\b(fkb\w+Timeouts)\(\)", body))
+
+
 def test_enum_values_and_strings(L):
     assert (fk.OP_N, fk.OP_T) == (1, 2)
     assert fk.BACKEND_CUDA == 8 and fk.BACKEND_X86 == 2
