@@ -31,11 +31,10 @@
 // one lane: with run-time descriptors a 128x64x16 MMA took 126-152 clocks, with immediate ones the passes no longer
 // notice twice the MMAs.
 //
-// Operands a bf16 split cannot hold (infinities, NaN, magnitudes from 2^127 or whose sums could overflow; rows or
-// factor columns that are tiny throughout, below 2^-90 or 2^-100 together, whose low parts would fall under the
-// smallest normal numbers) are found while
-// splitting: such a row, or every row when the factor is concerned, is recomputed by its epilogue thread as
-// the plain FMA chain over p.
+// Operands a bf16 split cannot hold are found while splitting: elements with a remainder after the third piece
+// (infinities, NaN, and numbers below about 2^-110 whose last bits lie under the smallest bf16 denormal 2^-133; the
+// tensor cores take and give denormals in full), and magnitudes from 2^127 or whose sums could overflow.  A row with such
+// an element, or every row when the factor has one, is recomputed by its epilogue thread as the plain FMA chain over p.
 #include <stdlib.h>
 
 #include <cuda_bf16.h>
@@ -56,11 +55,9 @@ constexpr int kSplitChunk = 16;                    // p per stage: a stage is 32
 constexpr int kSplitStageElems = 32 * kSplitChunk;
 constexpr int kSplitMaxStages = 5;
 constexpr int kSplitSmem = (227 - 3) * 1024;         // dynamic shared memory; the static part is below 3 KB
-constexpr unsigned kRowHuge = 1, kRowNormal = 2, kRowNonzero = 4;
 constexpr int kXposePitch = 36;                    // 32 columns and an odd number of 16-byte units per row
 constexpr size_t kXposeBytes = kSplitEpiWarps * 32 * kXposePitch * sizeof(float);
 constexpr unsigned kHuge = 254u << 23;             // 2^127 as float bits
-constexpr unsigned kTiny = 37u << 23;              // 2^-90
 
 struct SplitArgs {
   const float* X; float* Z; const float* Y; const float* F;
@@ -128,15 +125,18 @@ __device__ __forceinline__ void mmaBf16TmemA(unsigned elected, unsigned d, unsig
       ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
 }
 
-// Two neighbouring values of the contraction index as packed bf16 pairs (x0 in the low half).
-__device__ __forceinline__ void split2(float x0, float x1, unsigned& h, unsigned& m, unsigned& l) {
+// Two neighbouring values of the contraction index as packed bf16 pairs (x0 in the low half).  Returns 0 when h + m + l
+// is x for both, something else when a remainder is left or a value is not finite.
+__device__ __forceinline__ unsigned split2(float x0, float x1, unsigned& h, unsigned& m, unsigned& l) {
   const __nv_bfloat162 hp = __floats2bfloat162_rn(x0, x1);
   const float r0 = x0 - __low2float(hp), r1 = x1 - __high2float(hp);          // exact
   const __nv_bfloat162 mp = __floats2bfloat162_rn(r0, r1);
-  const __nv_bfloat162 lp = __floats2bfloat162_rn(r0 - __low2float(mp), r1 - __high2float(mp));
+  const float s0 = r0 - __low2float(mp), s1 = r1 - __high2float(mp);          // exact
+  const __nv_bfloat162 lp = __floats2bfloat162_rn(s0, s1);
   h = *reinterpret_cast<const unsigned*>(&hp);
   m = *reinterpret_cast<const unsigned*>(&mp);
   l = *reinterpret_cast<const unsigned*>(&lp);
+  return __float_as_uint(s0 - __low2float(lp)) | __float_as_uint(s1 - __high2float(lp));
 }
 
 // XT: the contracted index is contiguous in X (lanes load along p); otherwise lanes load along j.
@@ -154,10 +154,9 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   __shared__ __align__(8) unsigned long long aFull[2], aEmpty[2], dFull[2], dEmpty[2];
   __shared__ unsigned tmemBaseSlot;
   __shared__ int abortFlag, factorSpecial;
-  __shared__ unsigned rowHuge, rowTiny;
-  __shared__ unsigned factorMax, factorMin;                 // float bits: largest and smallest nonzero column maximum
-  __shared__ unsigned colMax[128];
-  __shared__ unsigned char rowState[4][2][kSplitRows];       // kRow* flags of a position, from its two converter warps
+  __shared__ unsigned rowHuge;
+  __shared__ unsigned factorMax;                             // float bits of the largest magnitude
+  __shared__ unsigned char rowState[4][2][kSplitRows];       // 1: the position's row cannot be split; from its two converter warps
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   constexpr unsigned aCols = 3 * half;                     // TMEM columns of one A buffer: [h][m][l]
@@ -167,57 +166,46 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   if (tid == 0) {
     for (int i = 0; i < 2; i++) { mbarInit(&aFull[i], kSplitConvWarps / 2); mbarInit(&aEmpty[i], 1); mbarInit(&dFull[i], 1); mbarInit(&dEmpty[i], kSplitEpiWarps); }
     abortFlag = 0; factorSpecial = 0;
-    factorMax = 0; factorMin = kHuge;
+    factorMax = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
   if (warp == kSplitMmaWarp) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(smemAddr(&tmemBaseSlot)), "r"(512) : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
-  if (tid < 128) colMax[tid] = 0;
   __syncthreads();
   // factor -> three bf16 copies, row q, k contiguous: 16-byte unit (k % 64) / 8 XOR (q % 8)
-  auto putFactor = [&](unsigned kp, unsigned q) -> unsigned {
+  unsigned fMax = 0, fLeft = 0;
+  auto putFactor = [&](unsigned kp, unsigned q) {
     const unsigned k = 2 * kp;
     const bool okQ = q < a.Q;
     const float* f = a.F + (long long)k * a.fsP + (long long)q * a.fsQ;
     const float v0 = okQ && k < a.P ? f[0] : 0.f, v1 = okQ && k + 1 < a.P ? f[a.fsP] : 0.f;
     unsigned h, m, l;
-    split2(v0, v1, h, m, l);
+    fLeft |= split2(v0, v1, h, m, l);
+    fMax = max(fMax, max(__float_as_uint(v0) & 0x7FFFFFFFu, __float_as_uint(v1) & 0x7FFFFFFFu));
     unsigned char* d = Fs + (k >> 6) * (a.N * 128u) + q * 128u + ((((k & 63) >> 3) ^ (q & 7)) << 4) + (k & 7) * 2u;
     *reinterpret_cast<unsigned*>(d) = h;
     *reinterpret_cast<unsigned*>(d + pieceBytes) = m;
     *reinterpret_cast<unsigned*>(d + 2 * pieceBytes) = l;
-    return max(__float_as_uint(v0) & 0x7FFFFFFFu, __float_as_uint(v1) & 0x7FFFFFFFu);
   };
   if (a.fsP != 1 || a.fsQ == 1) {
     for (unsigned kp = warp; kp < K / 2; kp += kSplitThreads / 32)
-      for (unsigned q = lane; q < a.N; q += 32) atomicMax(&colMax[q], putFactor(kp, q));
+      for (unsigned q = lane; q < a.N; q += 32) putFactor(kp, q);
   } else {
-    for (unsigned q = warp; q < a.N; q += kSplitThreads / 32) {
-      unsigned mx = 0;
-      for (unsigned kp = lane; kp < K / 2; kp += 32) mx = max(mx, putFactor(kp, q));
-      mx = __reduce_max_sync(0xffffffffu, mx);
-      if (lane == 0) colMax[q] = mx;
-    }
+    for (unsigned q = warp; q < a.N; q += kSplitThreads / 32)
+      for (unsigned kp = lane; kp < K / 2; kp += 32) putFactor(kp, q);
   }
+  fMax = __reduce_max_sync(0xffffffffu, fMax);
+  if (lane == 0) atomicMax(&factorMax, fMax);
+  if (fLeft != 0 || fMax >= kHuge) factorSpecial = 1;
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");      // generic-proxy writes -> tensor-core reads
   fenceBeforeSync();
   __syncthreads();
   fenceAfterSync();
-  if (tid < 128) {
-    const unsigned c = colMax[tid];
-    if (c >= kHuge || (c != 0 && c < kTiny)) factorSpecial = 1;
-    atomicMax(&factorMax, c);
-    if (c != 0) atomicMin(&factorMin, c);
-  }
-  __syncthreads();
-  if (tid == 0) {
-    // row magnitudes at which a sum of 128 products may pass 2^126 (terms of a split could become infinities of
-    // opposite signs) or the low terms of a column fall below the normal numbers
-    rowHuge = min(kHuge, __float_as_uint(0x1p119f / __uint_as_float(factorMax)));
-    rowTiny = max(kTiny, __float_as_uint(0x1p-100f / __uint_as_float(factorMin)));
-  }
+  // the row magnitude at which a sum of 128 products may pass 2^126 (terms of a split could become infinities of
+  // opposite signs)
+  if (tid == 0) rowHuge = min(kHuge, __float_as_uint(0x1p119f / __uint_as_float(factorMax)));
   __syncthreads();
   const unsigned tmemBase = *(volatile unsigned*)&tmemBaseSlot;
   volatile int* abortP = &abortFlag;
@@ -244,8 +232,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
       fenceAfterSync();
-      const unsigned state = rowState[it & 3][0][quarter * 32 + lane] | rowState[it & 3][1][quarter * 32 + lane];
-      const bool special = live && (allSpecial || (state & kRowHuge) != 0 || (state & (kRowNormal | kRowNonzero)) == kRowNonzero);
+      const bool special = live && (allSpecial || (rowState[it & 3][0][quarter * 32 + lane] | rowState[it & 3][1][quarter * 32 + lane]) != 0);
       const bool store = live && !special;
       const unsigned tcol = dCol + d * dCols + ((quarter * 32u) << 16);
 #pragma unroll 1
@@ -462,7 +449,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
       if (!ok) break;
       fenceAfterSync();
       __nv_bfloat162 mx = __floats2bfloat162_rn(0.f, 0.f);
-      unsigned any = 0;
+      unsigned left = 0;
 #pragma unroll 1
       for (unsigned c = sub; c < ks; c += 2) {
         cpAsyncWaitUpTo(a.stages - 1);
@@ -485,18 +472,16 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
         unsigned h[8], m[8], l[8];
 #pragma unroll
         for (int i = 0; i < 8; i++) {
-          split2(x[2 * i], x[2 * i + 1], h[i], m[i], l[i]);
-          mx = __hmax2_nan(mx, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&h[i])));
-          any |= __float_as_uint(x[2 * i]) | __float_as_uint(x[2 * i + 1]);
+          left |= split2(x[2 * i], x[2 * i + 1], h[i], m[i], l[i]);
+          mx = __hmax2(mx, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&h[i])));
         }
         const unsigned col = aBase + c * 8u;
         tmemStore8(col, h);
         tmemStore8(col + half, m);
         tmemStore8(col + 2 * half, l);
       }
-      const unsigned bits = __float_as_uint(__bfloat162float(__hmax_nan(__low2bfloat16(mx), __high2bfloat16(mx))));
-      rowState[(2 * li + group) & 3][sub][quarter * 32 + lane] =
-          (unsigned char)((bits >= rowHuge ? kRowHuge : 0u) | (bits >= rowTiny ? kRowNormal : 0u) | ((any << 1) != 0 ? kRowNonzero : 0u));
+      const unsigned bits = __float_as_uint(__bfloat162float(__hmax(__low2bfloat16(mx), __high2bfloat16(mx))));
+      rowState[(2 * li + group) & 3][sub][quarter * 32 + lane] = left != 0 || bits >= rowHuge ? 1 : 0;
       tmemStoreWait();
       fenceBeforeSync();
       __syncwarp();

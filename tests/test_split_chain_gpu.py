@@ -178,6 +178,32 @@ def test_split_pass_at_the_ends_of_the_range(lib, xs, fs):
     assert np.all(err <= 2.0 ** -24 * (P + 8) * (xn @ fn) + P * 2.0 ** -149)
 
 
+@pytest.mark.parametrize("small_in", ["x", "f"])
+def test_split_pass_keeps_small_elements_beside_large_ones(lib, small_in):
+    """Every output depends on one element of each operand (one nonzero per factor column), elements of one row or column
+    lie up to 2^149 apart, and the large partner brings the product back into the range: no output may lose bits
+    because its own element is small beside others of the same row or column.  One product: the bound of check()."""
+    import torch
+    import fastkron_b200
+    rng = np.random.default_rng(7)
+    M, P, Q = 1100, 64, 48
+    x = (rng.uniform(1, 2, (M, P)) * 10.0 ** rng.uniform(-45, 0, (M, P))).astype(np.float32)
+    f = np.zeros((P, Q), np.float32)
+    f[rng.permutation(P)[:Q], np.arange(Q)] = (rng.uniform(1, 2, Q) * 2.0 ** rng.integers(60, 110, Q)).astype(np.float32)
+    x[:, 0] = 1.0                                       # an ordinary element in every row
+    x[::2, 1:] = rng.uniform(-1, 1, (M // 2, P - 1))    # and rows that a split holds, beside the others in a tile
+    x[5, 1], f[1, 3] = 1.23456e-38, 1e33
+    x[7, 2], f[2, 4] = 2.0 ** -135, 2.0 ** 100
+    if small_in == "f":                                 # the mirror case: the same product with the roles exchanged
+        x, f = np.ascontiguousarray(np.resize(f.T, (M, P))), np.ascontiguousarray(x[:Q].T)
+    n0 = lib.fkbGemmSplitLaunches()
+    z = fastkron_b200.gemkm(torch.from_numpy(x).cuda(), [torch.from_numpy(f).cuda()]).cpu().numpy().astype(np.float64)
+    assert lib.fkbGemmSplitLaunches() == n0 + 1
+    xn, fn = x.astype(np.float64), f.astype(np.float64)
+    err, mag = np.abs(z - xn @ fn), np.abs(xn) @ np.abs(fn)
+    assert np.all(err <= 2.0 ** -24 * (P + 8) * mag + P * 2.0 ** -149), np.max(err / np.maximum(mag, 1e-300))
+
+
 CHAIN = [
     (1, [10] * 5, [10] * 5), (5, [12] * 4, [12] * 4), (300, [5] * 4, [5] * 4), (3, [14, 19, 34, 21], [15, 13, 23, 34]),
     (1, [2] * 9, [2] * 9), (64, [3, 7], [9, 2]), (7, [32, 9, 5], [11, 31, 6]), (2, [1, 6, 1, 5], [3, 1, 2, 4]),
