@@ -1,35 +1,43 @@
-// Large-factor pass of fp32 operands on the tensor cores with fp32 results: every operand is split
-// EXACTLY into three bf16 numbers, v = h + m + l (8 + 8 + 8 significant bits hold the 24 of a float),
-// and a product is formed as  h*h + (h*m + m*h) + (m*m + h*l + l*h)  with fp32 accumulation.  The three
-// terms left out (m*l, l*m, l*l) are below 2^-26 of the product; the six kept ones are exact in the
-// multiplier, so what remains is the rounding of the accumulator, once per 16 products instead of once per
-// product as in an FMA chain.  The small terms are accumulated first, so that only the P/16 steps of h*h
-// round at the magnitude of the result.
+// Large-factor pass of fp32 operands on the tensor cores with fp32 results.  Every operand is split into three bf16
+// numbers, v = h + m + l with 6, 8 and the remaining bits, which hold all 24 of a float, and the eight products of pieces
+// down to m*l and l*m are accumulated by tcgen05.mma (l*l, below 2^-30 of the product, is left out).
+//
+// The tensor cores cut every addend off two bits below the accumulator and every sum at 24 bits, both toward zero, so a sum
+// of one sign loses on average half a unit in the last place per step, always in the same direction and adding up over the
+// factors of a call.  Three things keep that out of the results:
+//   h has 6 bits only: products of two have 12, and a few of them add up without anything to cut off;
+//   h*h is summed in accumulators of 32 products each, which the epilogue adds with rounding to nearest;
+//   the other seven products, at most 2^-5 of the whole together, have an accumulator of their own, added last.
+// Error against 64-bit arithmetic (relative 2-norm, B200) of the FMA kernels and here: 64x64 twice 2.0e-7 and 4.2e-8 on values
+// in [-1, 1), 1.15e-7 and 3.1e-8 on [0, 1); 127x127 twice 2.9e-7 and 5.1e-8, 1.6e-7 and 3.7e-8.  It is larger than theirs only where
+// products of one sign spread over many magnitudes (lognormal values with sigma 2 and more, 1.0 to 3.7 times): the bits of
+// the small ones beside the large are still cut.
 //
 // One pass is  Z[j][q] = sum_p X[j][p] * F[p][q]  over the J = M*A*B positions (m, a, b) of the pass,
-// any strides, any P and Q up to 128, any alignment.  A tile is 128 positions times all of Q:
-//   D[128 x Q] (TMEM, fp32) += A[128 x P] (TMEM, bf16) * B[P x Q] (shared memory, bf16),  tcgen05.mma.kind::f16.
+// any strides, any P and Q up to 128, any alignment.  A tile is 128 positions times all of Q, in blocks of 64 columns:
+//   D[128 x 64] (TMEM, fp32) += A[128 x P] (TMEM, bf16) * B[P x 64] (shared memory, bf16),  tcgen05.mma.kind::f16.
 // Why A sits in TMEM: the positions come with j contiguous (B > 1) or p contiguous (B == 1), at any
 // alignment.  A converter thread owns one position: it reads its P values from shared memory, splits them in
 // registers and writes them to its TMEM lane with tcgen05.st.  The transposition that the j-contiguous
 // operand needs happens on that way for nothing, and the tensor cores read X without touching shared
 // memory (with the three copies there, operand reads alone would take as long as the HBM transfer).
 //
-// Warp roles (800 threads, one CTA per SM, persistent):
-//   0-7   epilogue: tcgen05.ld of the accumulator (a lane quarter each, alternate groups of 32 columns),
+// Warp roles (672 threads, one CTA per SM, persistent):
+//   0-7   epilogue: tcgen05.ld of the accumulators (a lane quarter each, alternate groups of 32 columns), their sum,
 //         alpha / beta*Y, stores
-//   8-23  converters, two groups of eight warps that take alternate tiles.  Two warps share 32 positions and
-//         take alternate chunks of 16 p; each loads its chunks with cp.async into a private ring of stages, so
-//         between load and conversion there is no barrier, only a __syncwarp
-//   24    MMA issue and the TMEM allocation.  The whole warp walks the loop (its values then stay in uniform
+//   8-19  converters.  Three warps share 32 positions and take the chunks of 16 p, tile after tile, in turns; each loads its
+//         chunks with cp.async into a private ring of stages, so between load and conversion there is no barrier, only a
+//         __syncwarp
+//   20    MMA issue and the TMEM allocation.  The whole warp walks the loop (its values then stay in uniform
 //         registers, where the instruction wants them) and one elected lane issues
-// Every wait on a barrier is bounded; one that gives up raises the abort flag that ends all roles.
+// A is handed over chunk by chunk: the MMAs of a chunk, all eight products, follow its conversion, and its place in
+// TMEM is free again when they are done.  Accumulators are two rings, h*h and the rest.
+// Every wait on a barrier is bounded; one that gives up raises the abort flag that ends all roles.  21 warps leave 80 registers a
+// thread, the fewest with which nothing is spilled (25 warps: 72, and with all of the SM's memory taken as shared memory
+// a spilled register comes back from L2: 64x64 four times, 64 rows, 9.3 ms against 8.5).
 //
-// Bound by HBM traffic and, where P is small, by the fixed work of a tile.  Measured on B200, 268 MB in and out (81 us at the copy
-// rate), 64x64: 97 us a pass with j contiguous (FMA kernel 187), 127 us with p contiguous (cold X; 59 against 85 us at
-// 100 MB); 128x128 and 134 MB (40 us): 64 / 74 us (FMA 320).  The contraction length is a template parameter because the MMAs are issued by
-// one lane: with run-time descriptors a 128x64x16 MMA took 126-152 clocks, with immediate ones the passes no longer
-// notice twice the MMAs.
+// Bound by issue slots (60 % busy) and by the hand-overs between the roles.  The contraction length is a template parameter
+// because the MMAs are issued by one lane: with run-time descriptors a 128x64x16 MMA took 126-152 clocks.
 //
 // Operands a bf16 split cannot hold are found while splitting: elements with a remainder after the third piece
 // (infinities, NaN, and numbers below about 2^-110 whose last bits lie under the smallest bf16 denormal 2^-133; the
@@ -47,17 +55,34 @@
 namespace fkb {
 namespace tc {
 
-constexpr int kSplitEpiWarps = 8, kSplitConvWarps = 16;
+constexpr int kSplitEpiWarps = 8, kSplitConvWarps = 12, kSplitSubs = kSplitConvWarps / 4;
 constexpr int kSplitMmaWarp = kSplitEpiWarps + kSplitConvWarps;
 constexpr int kSplitThreads = 32 * (kSplitMmaWarp + 1);
 constexpr int kSplitRows = 128;
 constexpr int kSplitChunk = 16;                    // p per stage: a stage is 32 positions x 16 p of one converter warp
 constexpr int kSplitStageElems = 32 * kSplitChunk;
-constexpr int kSplitMaxStages = 5;
+constexpr int kSplitMaxStages = 8;
 constexpr int kSplitSmem = (227 - 3) * 1024;         // dynamic shared memory; the static part is below 3 KB
 constexpr int kXposePitch = 36;                    // 32 columns and an odd number of 16-byte units per row
 constexpr size_t kXposeBytes = kSplitEpiWarps * 32 * kXposePitch * sizeof(float);
+constexpr unsigned kBlockN = 64;                   // columns of an accumulator: wider results go in blocks of 64
+// Steps of 16 products of h*h that share an accumulator.  With four, smooth one-signed factors (exp(-|i-j|/3)) err more than in
+// the FMA chain (3.7e-7 against 1.7e-7, 64x64 twice); with one the epilogue reads twice as many (64x64: 10.0 ms against 8.9).
+constexpr unsigned kHhSteps = 2;
+// A buffers: from P = 81 on the accumulators leave room for one.
+__host__ __device__ constexpr unsigned aBuffers(unsigned ks) { return ks > 5 ? 1 : 2; }
+constexpr unsigned kMaxSlots = 8;                  // accumulators
 constexpr unsigned kHuge = 254u << 23;             // 2^127 as float bits
+
+// n / d for n < 2^31:  n * ceil(2^(31+l) / d) >> (31 + l), l = ceil(log2 d); the factor fits 32 bits (m == 0: d is 1).
+struct PosDiv { unsigned d, m, s; };
+static PosDiv posDiv(unsigned d) {
+  unsigned l = 0;
+  while ((1ull << l) < d) l++;
+  if (l == 0) return PosDiv{1, 0, 0};
+  return PosDiv{d, (unsigned)(((1ull << (31 + l)) + d - 1) / d), l - 1};
+}
+__device__ __forceinline__ unsigned quot(unsigned n, const PosDiv& f) { return f.m == 0 ? n : __umulhi(n, f.m) >> f.s; }
 
 struct SplitArgs {
   const float* X; float* Z; const float* Y; const float* F;
@@ -65,10 +90,11 @@ struct SplitArgs {
   unsigned P, Q;
   unsigned N;                                      // Q rounded up to 16
   unsigned stages;                                 // per converter warp, 1 .. kSplitMaxStages
+  unsigned slotCols, sSlots, slots;                // TMEM columns of an accumulator; 0 .. sSlots-1 take small terms, sSlots .. slots-1 h*h, each a ring
   // position J = (i2*n1 + i1)*n0 + i0; element (J, p) of X at sum i*xs + p*xsP, (J, q) of Z and Y at sum i*zs + q*zsQ
-  unsigned n0, n1;
-  long long xs0, xs1, xs2, xsP;
-  long long zs0, zs1, zs2, zsQ;
+  PosDiv n0, n1;
+  unsigned xs0, xs1, xs2, zs0, zs1, zs2;           // elements
+  long long xsP, zsQ;
   unsigned total, numTiles;
   float alpha, beta;
   int epilogue;
@@ -104,7 +130,10 @@ __device__ __forceinline__ void cpAsyncWaitUpTo(unsigned n) {
     case 1: asm volatile("cp.async.wait_group 1;\n" ::: "memory"); break;
     case 2: asm volatile("cp.async.wait_group 2;\n" ::: "memory"); break;
     case 3: asm volatile("cp.async.wait_group 3;\n" ::: "memory"); break;
-    default: asm volatile("cp.async.wait_group 4;\n" ::: "memory"); break;
+    case 4: asm volatile("cp.async.wait_group 4;\n" ::: "memory"); break;
+    case 5: asm volatile("cp.async.wait_group 5;\n" ::: "memory"); break;
+    case 6: asm volatile("cp.async.wait_group 6;\n" ::: "memory"); break;
+    default: asm volatile("cp.async.wait_group 7;\n" ::: "memory"); break;
   }
 }
 
@@ -125,18 +154,19 @@ __device__ __forceinline__ void mmaBf16TmemA(unsigned elected, unsigned d, unsig
       ::"r"(d), "r"(a), "l"(b), "r"(idesc), "r"(accumulate), "r"(elected) : "memory");
 }
 
-// Two neighbouring values of the contraction index as packed bf16 pairs (x0 in the low half).  Returns 0 when h + m + l
-// is x for both, something else when a remainder is left or a value is not finite.
-__device__ __forceinline__ unsigned split2(float x0, float x1, unsigned& h, unsigned& m, unsigned& l) {
-  const __nv_bfloat162 hp = __floats2bfloat162_rn(x0, x1);
-  const float r0 = x0 - __low2float(hp), r1 = x1 - __high2float(hp);          // exact
+// Two neighbouring values of the contraction index as packed bf16 pairs (x0 in the low half): h to 6 bits and m to 8, each
+// rounded to nearest, and what is left, l.  h + m + l is x (6 + 1 + 8 + 1 + 8 bits: a remainder rounded to nearest has one
+// bit less) unless l has bits below a bf16's, which the caller finds in the low half of `left`, as with values that are
+// not finite.
+__device__ __forceinline__ void split2(float x0, float x1, unsigned& h, unsigned& m, unsigned& l, unsigned& left) {
+  const unsigned h0 = (__float_as_uint(x0) + 0x20000u) & 0xFFFC0000u, h1 = (__float_as_uint(x1) + 0x20000u) & 0xFFFC0000u;
+  const float r0 = x0 - __uint_as_float(h0), r1 = x1 - __uint_as_float(h1);   // exact
   const __nv_bfloat162 mp = __floats2bfloat162_rn(r0, r1);
-  const float s0 = r0 - __low2float(mp), s1 = r1 - __high2float(mp);          // exact
-  const __nv_bfloat162 lp = __floats2bfloat162_rn(s0, s1);
-  h = *reinterpret_cast<const unsigned*>(&hp);
+  const unsigned l0 = __float_as_uint(r0 - __low2float(mp)), l1 = __float_as_uint(r1 - __high2float(mp));   // exact
+  h = __byte_perm(h0, h1, 0x7632);
   m = *reinterpret_cast<const unsigned*>(&mp);
-  l = *reinterpret_cast<const unsigned*>(&lp);
-  return __float_as_uint(s0 - __low2float(lp)) | __float_as_uint(s1 - __high2float(lp));
+  l = __byte_perm(l0, l1, 0x7632);
+  left |= l0 | l1;
 }
 
 // XT: the contracted index is contiguous in X (lanes load along p); otherwise lanes load along j.
@@ -145,26 +175,29 @@ template <bool XT, int KS>
 __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitArgs a) {
   constexpr unsigned K = 16 * KS, ks = KS, half = K / 2;     // half: TMEM columns of one piece of A
   constexpr unsigned slabs = (K + 63) / 64;
+  constexpr unsigned hSlots = (KS + kHhSteps - 1) / kHhSteps;  // accumulators of h*h per block of columns
   extern __shared__ unsigned char smemRaw[];
   unsigned char* base = reinterpret_cast<unsigned char*>(((uintptr_t)smemRaw + 1023) & ~(uintptr_t)1023);
   const unsigned pieceBytes = slabs * a.N * 128u;            // one bf16 copy of the factor: [K/64][N rows q][64 k], 128-byte swizzle
   unsigned char* Fs = base;
   float* xpose = reinterpret_cast<float*>(base + 3 * pieceBytes);                             // outT only
   float* ring = xpose + (a.outT ? kXposeBytes / sizeof(float) : 0);
-  __shared__ __align__(8) unsigned long long aFull[2], aEmpty[2], dFull[2], dEmpty[2];
+  __shared__ __align__(8) unsigned long long aFull[2][8], aEmpty[2][8], dFull[kMaxSlots], dEmpty[kMaxSlots], drained;
   __shared__ unsigned tmemBaseSlot;
   __shared__ int abortFlag, factorSpecial;
   __shared__ unsigned rowHuge;
   __shared__ unsigned factorMax;                             // float bits of the largest magnitude
-  __shared__ unsigned char rowState[4][2][kSplitRows];       // 1: the position's row cannot be split; from its two converter warps
+  __shared__ unsigned short rowState[8][kSplitRows];  // tile it, position: (it >> 3) + 1 if its row cannot be split
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  constexpr unsigned nA = aBuffers(KS);
   constexpr unsigned aCols = 3 * half;                     // TMEM columns of one A buffer: [h][m][l]
-  const unsigned dCols = (a.N + 31) & ~31u;                  // one accumulator (read back 32 columns at a time)
-  const unsigned nD = 2 * aCols + 2 * dCols <= 512 ? 2 : 1;  // accumulators; P, Q <= 128 leave room for one
 
   if (tid == 0) {
-    for (int i = 0; i < 2; i++) { mbarInit(&aFull[i], kSplitConvWarps / 2); mbarInit(&aEmpty[i], 1); mbarInit(&dFull[i], 1); mbarInit(&dEmpty[i], kSplitEpiWarps); }
+    for (int i = 0; i < 16; i++) { mbarInit(&aFull[i >> 3][i & 7], 4); mbarInit(&aEmpty[i >> 3][i & 7], 1); }
+    // dFull: the commit of the MMAs, and an ordinary arrival that carries what the converters wrote (rowState)
+    for (unsigned i = 0; i < kMaxSlots; i++) { mbarInit(&dFull[i], 2); mbarInit(&dEmpty[i], kSplitEpiWarps); }
+    mbarInit(&drained, 1);
     abortFlag = 0; factorSpecial = 0;
     factorMax = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
@@ -174,6 +207,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   __syncthreads();
+  for (unsigned i = tid; i < 8 * kSplitRows; i += kSplitThreads) (&rowState[0][0])[i] = 0;
   // factor -> three bf16 copies, row q, k contiguous: 16-byte unit (k % 64) / 8 XOR (q % 8)
   unsigned fMax = 0, fLeft = 0;
   auto putFactor = [&](unsigned kp, unsigned q) {
@@ -182,7 +216,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     const float* f = a.F + (long long)k * a.fsP + (long long)q * a.fsQ;
     const float v0 = okQ && k < a.P ? f[0] : 0.f, v1 = okQ && k + 1 < a.P ? f[a.fsP] : 0.f;
     unsigned h, m, l;
-    fLeft |= split2(v0, v1, h, m, l);
+    split2(v0, v1, h, m, l, fLeft);
     fMax = max(fMax, max(__float_as_uint(v0) & 0x7FFFFFFFu, __float_as_uint(v1) & 0x7FFFFFFFu));
     unsigned char* d = Fs + (k >> 6) * (a.N * 128u) + q * 128u + ((((k & 63) >> 3) ^ (q & 7)) << 4) + (k & 7) * 2u;
     *reinterpret_cast<unsigned*>(d) = h;
@@ -198,7 +232,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   }
   fMax = __reduce_max_sync(0xffffffffu, fMax);
   if (lane == 0) atomicMax(&factorMax, fMax);
-  if (fLeft != 0 || fMax >= kHuge) factorSpecial = 1;
+  if ((fLeft & 0xFFFFu) != 0 || fMax >= kHuge) factorSpecial = 1;
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");      // generic-proxy writes -> tensor-core reads
   fenceBeforeSync();
   __syncthreads();
@@ -209,7 +243,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   __syncthreads();
   const unsigned tmemBase = *(volatile unsigned*)&tmemBaseSlot;
   volatile int* abortP = &abortFlag;
-  const unsigned dCol = tmemBase + 2 * aCols;
+  const unsigned dCol = tmemBase + nA * aCols;
 
   const unsigned first = blockIdx.x, step = gridDim.x;
   const unsigned myTiles = first < a.numTiles ? (a.numTiles - first + step - 1) / step : 0;
@@ -220,43 +254,73 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     const bool epi = a.epilogue != 0;
     const bool useY = epi && a.beta != 0.f && a.Y != nullptr;
     const bool allSpecial = factorSpecial != 0;
-    const bool linear = a.n0 == a.total;
+    const bool linear = a.n0.d == a.total;
     float* sc = xpose + warp * 32 * kXposePitch;
-    for (unsigned it = 0; it < myTiles; it++) {
-      const unsigned d = nD == 2 ? (it & 1u) : 0u, use = nD == 2 ? (it >> 1) : it;
+    // take(): the MMAs into accumulator `sl` are complete; give(): this warp has read it.  Each set has full-barriers of
+    // its own (a wait for a later phase than the next is none); bit `sl` of phases: parity of the next one of `sl`.
+    unsigned sSlot = 0, slot = a.sSlots, phases = 0;
+    auto take = [&](unsigned sl) {
+      const bool all = __all_sync(0xffffffffu, waitBounded(&dFull[sl], phases >> sl & 1u, abortP));
+      phases ^= 1u << sl;
+      fenceAfterSync();
+      return all;
+    };
+    auto give = [&](unsigned sl) {
+      fenceBeforeSync();
+      __syncwarp();
+      if (lane == 0) mbarArrive(&dEmpty[sl]);
+    };
+    bool alive = true;
+    for (unsigned it = 0; alive && it < myTiles; it++) {
       const unsigned J = (first + it * step) * (unsigned)kSplitRows + quarter * 32u + (unsigned)lane;
       const bool live = J < a.total;
-      const unsigned r0 = J / a.n0, i0 = J - r0 * a.n0, i2 = r0 / a.n1, i1 = r0 - i2 * a.n1;
-      const long long zoff = (long long)i0 * a.zs0 + (long long)i1 * a.zs1 + (long long)i2 * a.zs2;
-      bool ok = !*abortP && waitBounded(&dFull[d], use & 1u, abortP);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      fenceAfterSync();
-      const bool special = live && (allSpecial || (rowState[it & 3][0][quarter * 32 + lane] | rowState[it & 3][1][quarter * 32 + lane]) != 0);
-      const bool store = live && !special;
-      const unsigned tcol = dCol + d * dCols + ((quarter * 32u) << 16);
+      const unsigned r0 = quot(J, a.n0), i0 = J - r0 * a.n0.d, i2 = quot(r0, a.n1), i1 = r0 - i2 * a.n1.d;
+      const long long zoff = (long long)((unsigned long long)i0 * a.zs0 + (unsigned long long)i1 * a.zs1 + (unsigned long long)i2 * a.zs2);
+      bool special = false, store = false;
 #pragma unroll 1
-      for (unsigned c0 = part * 32u; c0 < a.N || c0 < 64u; c0 += 64) {
-        unsigned r[32];
-        if (c0 < a.N) {
-          tmemLoad32(tcol + c0, r);
-          tmemLoadWait();
+      for (unsigned cb = 0; cb < a.N; cb += kBlockN) {
+        const unsigned c0 = cb + part * 32u;
+        const unsigned tcol = dCol + part * 32u + ((quarter * 32u) << 16);
+        float r[32];
+        // h*h first, then the small terms: one rounding to nearest per accumulator
+        auto addFrom = [&](unsigned sl) {
+#pragma unroll
+          for (unsigned g = 0; g < 32; g += 16) {
+            unsigned t[16];
+            tmemLoad16(tcol + sl * a.slotCols + g, t);
+            tmemLoadWait();
+#pragma unroll
+            for (unsigned i = 0; i < 16; i++) r[g + i] += __uint_as_float(t[i]);
+          }
+        };
+#pragma unroll 1
+        for (unsigned h = 0; h < hSlots; h++) {
+          if (!take(slot)) { alive = false; break; }
+          if (c0 < a.N) {
+            if (h == 0) { tmemLoad32(tcol + slot * a.slotCols, reinterpret_cast<unsigned(&)[32]>(r)); tmemLoadWait(); }
+            else addFrom(slot);
+          }
+          give(slot);
+          if (++slot == a.slots) slot = a.sSlots;
         }
-        if (c0 + 64 >= a.N) {                                 // accumulator fully read: hand it back
-          fenceBeforeSync();
-          __syncwarp();
-          if (lane == 0) mbarArrive(&dEmpty[d]);
+        if (!alive || !take(sSlot)) { alive = false; break; }
+        if (cb == 0) {
+          special = live && (allSpecial || rowState[it & 7][quarter * 32 + lane] == (unsigned short)((it >> 3) + 1u));
+          store = live && !special;
         }
+        if (c0 < a.N) addFrom(sSlot);
+        give(sSlot);
+        if (++sSlot == a.sSlots) sSlot = 0;
         if (!a.outT) {
           float* z = a.Z + zoff + (long long)c0 * a.zsQ;
           if (!epi) {
             if (store && c0 + 32 <= a.Q) {
 #pragma unroll
-              for (unsigned i = 0; i < 32; i++, z += a.zsQ) *z = __uint_as_float(r[i]);
+              for (unsigned i = 0; i < 32; i++, z += a.zsQ) *z = r[i];
             } else if (store) {
 #pragma unroll
               for (unsigned i = 0; i < 32; i++, z += a.zsQ)
-                if (c0 + i < a.Q) *z = __uint_as_float(r[i]);
+                if (c0 + i < a.Q) *z = r[i];
             }
           } else if (store) {
             const float* y = a.Y + zoff + (long long)c0 * a.zsQ;
@@ -267,7 +331,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
               for (unsigned i = 0; i < 4; i++) yv[i] = useY && c0 + g + i < a.Q ? y[(long long)(g + i) * a.zsQ] : 0.f;
 #pragma unroll
               for (unsigned i = 0; i < 4; i++, z += a.zsQ) {
-                float v = a.alpha * __uint_as_float(r[g + i]);
+                float v = a.alpha * r[g + i];
                 if (useY) v = fmaf(a.beta, yv[i], v);
                 if (c0 + g + i < a.Q) *z = v;
               }
@@ -279,11 +343,11 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
           const unsigned stores = __ballot_sync(0xffffffffu, store);
 #pragma unroll
           for (unsigned i = 0; i < 32; i += 4)
-            *reinterpret_cast<uint4*>(sc + lane * kXposePitch + i) = make_uint4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+            *reinterpret_cast<float4*>(sc + lane * kXposePitch + i) = make_float4(r[i], r[i + 1], r[i + 2], r[i + 3]);
           __syncwarp();
           // offset of row rr of this warp's 32, also on lanes whose own position lies beyond the last
           auto rowOff = [&](unsigned rr) -> long long {
-            if (linear) return (long long)(J - (unsigned)lane + rr) * a.zs0;
+            if (linear) return (long long)((unsigned long long)(J - (unsigned)lane + rr) * a.zs0);
             return __shfl_sync(0xffffffffu, zoff, (int)rr);
           };
           // (reads of a batch of rows ahead of their stores: a store may alias the scratch as far as the compiler knows)
@@ -334,8 +398,8 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
           __syncwarp();
         }
       }
-      if (special && part == 0) {
-        const float* x = a.X + (long long)i0 * a.xs0 + (long long)i1 * a.xs1 + (long long)i2 * a.xs2;
+      if (alive && special && part == 0) {
+        const float* x = a.X + (unsigned long long)i0 * a.xs0 + (unsigned long long)i1 * a.xs1 + (unsigned long long)i2 * a.xs2;
         for (unsigned q = 0; q < a.Q; q++) {
           float acc = 0.f;
           for (unsigned p = 0; p < a.P; p++) acc = fmaf(x[(long long)p * a.xsP], a.F[(long long)p * a.fsP + (long long)q * a.fsQ], acc);
@@ -348,26 +412,28 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   } else if (warp < kSplitMmaWarp) {
     // ---- converters ----------------------------------------------------------------------------
     const unsigned cw = (unsigned)(warp - kSplitEpiWarps);
-    const unsigned group = cw >> 3, sub = (cw >> 2) & 1u, quarter = cw & 3u;
+    const unsigned sub = cw >> 2, quarter = cw & 3u;
     constexpr unsigned stageBytes = kSplitStageElems * 4;
     const unsigned myRing = smemAddr(ring) + cw * a.stages * stageBytes;
-    // this warp takes the chunks sub, sub + 2, ... of the ks
-    const unsigned myGroupTiles = ks > sub && myTiles > group ? (myTiles - group + 1) / 2 : 0;
-    // the loads run ahead of the conversion by the depth of the ring: tile ldTile (of this group), chunk ldC
-    unsigned ldTile = 0, ldC = sub, ldMask = 0;
+    // The chunks of this CTA's tiles, one after the other, go round the three warps of a quarter.  The loads run ahead of
+    // the conversion by the depth of the ring: chunk ldN.
+    const unsigned chunks = myTiles * ks;
+    unsigned ldN = sub, ldTile = ~0u, ldMask = 0;
     // Input offsets of what this lane fetches, once per tile: ldOff of the position along j (the first of four with
     // 16-byte loads), or, with lanes along p, of position `lane`; ldRow, 16-byte loads along p: of the rows
     // lane / 4 + 8 i, in units of 16 bytes.  ldMask: which of them exist.
     long long ldOff = 0;
     unsigned ldRow[XT ? 4 : 1];
     auto offsetOf = [&](unsigned J) {
-      const unsigned r0 = J / a.n0, i0 = J - r0 * a.n0, i2 = r0 / a.n1, i1 = r0 - i2 * a.n1;
-      return (long long)i0 * a.xs0 + (long long)i1 * a.xs1 + (long long)i2 * a.xs2;
+      const unsigned r0 = quot(J, a.n0), i0 = J - r0 * a.n0.d, i2 = quot(r0, a.n1), i1 = r0 - i2 * a.n1.d;
+      return (long long)((unsigned long long)i0 * a.xs0 + (unsigned long long)i1 * a.xs1 + (unsigned long long)i2 * a.xs2);
     };
     auto load = [&](unsigned st) {
-      if (ldTile < myGroupTiles) {
-        if (ldC == sub) {
-          const unsigned J0 = (first + (2 * ldTile + group) * step) * (unsigned)kSplitRows + quarter * 32u;
+      if (ldN < chunks) {
+        const unsigned tile = ldN / ks;
+        if (tile != ldTile) {
+          ldTile = tile;
+          const unsigned J0 = (first + tile * step) * (unsigned)kSplitRows + quarter * 32u;
           const unsigned rows = a.total > J0 ? min(a.total - J0, 32u) : 0u;
           if constexpr (!XT) {
             const unsigned j = a.vecX ? (unsigned)(lane & 7) * 4u : (unsigned)lane;   // n0 % 4 == 0 with 16-byte loads: whole vectors
@@ -387,7 +453,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
             ldMask = rows;
           }
         }
-        const unsigned p0 = ldC * kSplitChunk;
+        const unsigned p0 = (ldN - tile * ks) * kSplitChunk;
         const bool whole = p0 + kSplitChunk <= a.P;     // else p beyond P: zeros
         if constexpr (!XT) {
           if (a.vecX) {
@@ -435,88 +501,114 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
             if (row < ldMask) cpAsyncFill<4>(st + row * 64 + ((((pl >> 2) ^ (row >> 1 & 3u)) << 4) | ((pl & 3u) << 2)), okP ? xp + ro : a.X, okP);
           }
         }
-        ldC += 2;
-        if (ldC >= ks) { ldC = sub; ldTile++; }
+        ldN += kSplitSubs;
       }
       asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
     for (unsigned s = 0; s < a.stages; s++) load(myRing + s * stageBytes);
     unsigned s = 0;
-    const unsigned aBase = tmemBase + group * aCols + ((quarter * 32u) << 16);
-    for (unsigned li = 0; li < myGroupTiles; li++) {
-      bool ok = !*abortP && waitBounded(&aEmpty[group], (li & 1u) ^ 1u, abortP);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      fenceAfterSync();
-      __nv_bfloat162 mx = __floats2bfloat162_rn(0.f, 0.f);
-      unsigned left = 0;
 #pragma unroll 1
-      for (unsigned c = sub; c < ks; c += 2) {
-        cpAsyncWaitUpTo(a.stages - 1);
-        __syncwarp();
-        const unsigned st = myRing + s * stageBytes;
-        float x[16];
-        if constexpr (!XT) {
+    for (unsigned n = sub; n < chunks; n += kSplitSubs) {
+      const unsigned it = n / ks, c = n - it * ks, g = it % nA;
+      cpAsyncWaitUpTo(a.stages - 1);
+      __syncwarp();
+      const unsigned st = myRing + s * stageBytes;
+      float x[16];
+      if constexpr (!XT) {
 #pragma unroll
-          for (int i = 0; i < 16; i++) x[i] = ldShared(st + i * 128 + 4 * lane);
-        } else {
+        for (int i = 0; i < 16; i++) x[i] = ldShared(st + i * 128 + 4 * lane);
+      } else {
 #pragma unroll
-          for (int i = 0; i < 4; i++) {
-            const float4 v = ldShared4(st + lane * 64 + ((i ^ (lane >> 1 & 3)) << 4));
-            x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
-          }
+        for (int i = 0; i < 4; i++) {
+          const float4 v = ldShared4(st + lane * 64 + ((i ^ (lane >> 1 & 3)) << 4));
+          x[4 * i] = v.x; x[4 * i + 1] = v.y; x[4 * i + 2] = v.z; x[4 * i + 3] = v.w;
         }
-        __syncwarp();                                         // the stage has been read by every lane
-        load(st);
-        if (++s == a.stages) s = 0;
-        unsigned h[8], m[8], l[8];
-#pragma unroll
-        for (int i = 0; i < 8; i++) {
-          left |= split2(x[2 * i], x[2 * i + 1], h[i], m[i], l[i]);
-          mx = __hmax2(mx, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&h[i])));
-        }
-        const unsigned col = aBase + c * 8u;
-        tmemStore8(col, h);
-        tmemStore8(col + half, m);
-        tmemStore8(col + 2 * half, l);
       }
-      const unsigned bits = __float_as_uint(__bfloat162float(__hmax(__low2bfloat16(mx), __high2bfloat16(mx))));
-      rowState[(2 * li + group) & 3][sub][quarter * 32 + lane] = left != 0 || bits >= rowHuge ? 1 : 0;
+      __syncwarp();                                         // the stage has been read by every lane
+      load(st);
+      if (++s == a.stages) s = 0;
+      unsigned h[8], m[8], l[8], left = 0;
+      float mx = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; i++) {
+        split2(x[2 * i], x[2 * i + 1], h[i], m[i], l[i], left);
+        mx = fmaxf(mx, fmaxf(fabsf(x[2 * i]), fabsf(x[2 * i + 1])));
+      }
+      // (the use before the last one of this chunk has been consumed: 3 chunks are fewer than the buffers hold)
+      if (!__all_sync(0xffffffffu, waitBounded(&aEmpty[g][c], (it / nA & 1u) ^ 1u, abortP))) break;
+      fenceAfterSync();
+      const unsigned col = tmemBase + g * aCols + c * 8u + ((quarter * 32u) << 16);
+      tmemStore8(col, h);
+      tmemStore8(col + half, m);
+      tmemStore8(col + 2 * half, l);
+      if ((left & 0xFFFFu) != 0 || __float_as_uint(mx) >= rowHuge) rowState[it & 7][quarter * 32 + lane] = (unsigned short)((it >> 3) + 1u);
       tmemStoreWait();
       fenceBeforeSync();
       __syncwarp();
-      if (lane == 0) mbarArrive(&aFull[group]);
+      if (lane == 0) mbarArrive(&aFull[g][c]);
     }
     asm volatile("cp.async.wait_group 0;\n" ::: "memory");
   } else {
     // ---- MMA issue -------------------------------------------------------------------------------
     const unsigned elected = electOne();
-    const unsigned idesc = splitInstrDesc(a.N);
     const unsigned long long bDesc = smemDesc(smemAddr(Fs), 16u, 1024u, kSwz128);
     const unsigned pieceUnits = pieceBytes >> 4, slabUnits = a.N * 8u;   // descriptor addresses are in 16-byte units
-    for (unsigned it = 0; it < myTiles; it++) {
-      const unsigned g = it & 1u, aUse = it >> 1;
-      const unsigned d = nD == 2 ? g : 0u, dUse = nD == 2 ? aUse : it;
-      bool ok = !*abortP && waitBounded(&aFull[g], aUse & 1u, abortP) && waitBounded(&dEmpty[d], (dUse & 1u) ^ 1u, abortP);
-      ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
-      fenceAfterSync();
-      const unsigned tA = g * aCols, tD = 2 * aCols + d * dCols;         // the allocation is all of TMEM, it starts at 0
-      // six sweeps over the contraction index, the small terms first: piece pa of X times piece pb of the factor
-#pragma unroll
-      for (int t = 0; t < 6; t++) {
-        constexpr unsigned pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
-#pragma unroll
-        for (unsigned k = 0; k < ks; k++)
-          mmaBf16TmemA(elected, tD, tA + pa[t] * half + k * 8u, bDesc + pb[t] * pieceUnits + (k >> 2) * slabUnits + (k & 3u) * 2u, idesc,
-                       t > 0 || k > 0 ? 1u : 0u);
-      }
+    unsigned sSlot = 0, sPhase = 1, slot = a.sSlots, phase = 1;
+    bool alive = true;
+    auto waitFor = [&](unsigned long long* bar, unsigned ph) {
+      if (alive) alive = __all_sync(0xffffffffu, waitBounded(bar, ph, abortP));
+    };
+    auto give = [&](unsigned sl) {
       if (elected) {
-        mmaCommit(&aEmpty[g]);
-        mmaCommit(&dFull[d]);
+        mmaCommit(&dFull[sl]);
+        mbarArrive(&dFull[sl]);
       }
       __syncwarp();
+    };
+    for (unsigned it = 0; alive && it < myTiles; it++) {
+      const unsigned g = it % nA, aPhase = it / nA & 1u;
+      const unsigned tA = g * aCols;                           // the allocation is all of TMEM, it starts at 0
+#pragma unroll 1
+      for (unsigned cb = 0; alive && cb < a.N; cb += kBlockN) {
+        const unsigned idesc = splitInstrDesc(min(a.N - cb, kBlockN));
+        const unsigned long long bBlock = bDesc + cb * 8u;     // rows of 128 bytes
+        const bool lastBlock = cb + kBlockN >= a.N;
+        const unsigned tS = nA * aCols + sSlot * a.slotCols;
+        waitFor(&dEmpty[sSlot], sPhase);
+        unsigned tH = 0;
+#pragma unroll
+        for (unsigned k = 0; k < ks; k++) {
+          if (cb == 0) waitFor(&aFull[g][k], aPhase);
+          if (k % kHhSteps == 0) {
+            waitFor(&dEmpty[slot], phase);
+            tH = nA * aCols + slot * a.slotCols;
+          }
+          if (!alive) break;
+          fenceAfterSync();
+          const unsigned long long bK = bBlock + (k >> 2) * slabUnits + (k & 3u) * 2u;
+          // piece pa of X times piece pb of the factor: h*h, and everything but it and l*l into the tile's small terms
+          mmaBf16TmemA(elected, tH, tA + k * 8u, bK, idesc, k % kHhSteps != 0 ? 1u : 0u);
+          if (k % kHhSteps == kHhSteps - 1 || k == ks - 1) {
+            give(slot);
+            if (++slot == a.slots) { slot = a.sSlots; phase ^= 1u; }
+          }
+#pragma unroll
+          for (int t = 0; t < 7; t++) {
+            constexpr unsigned pa[7] = {1, 2, 2, 0, 1, 1, 0}, pb[7] = {2, 1, 0, 2, 1, 0, 1};
+            mmaBf16TmemA(elected, tS, tA + pa[t] * half + k * 8u, bK + pb[t] * pieceUnits, idesc, t > 0 || k > 0 ? 1u : 0u);
+          }
+          if (lastBlock && elected) mmaCommit(&aEmpty[g][k]);
+          __syncwarp();
+        }
+        if (alive) give(sSlot);
+        if (++sSlot == a.sSlots) { sSlot = 0; sPhase ^= 1u; }
+      }
     }
+    // No MMA may be in flight when the tensor memory goes back, also after a wait that gave up; about two seconds at most.
+    if (elected) mmaCommit(&drained);
+    __syncwarp();
+    const long long t0 = clock64();
+    while (!mbarTryWait(&drained, 0u) && clock64() - t0 < 4000000000ll) {}
   }
 
   // ---- teardown: every role gets here (all waits are bounded); release TMEM ----------------------
@@ -586,9 +678,14 @@ fastKronError launchGemmSplit(const Pass& ps, const LaunchCtx& cx) {
   a.outT = ps.zsG == 1 ? 1 : 0;
   PosDim d[3];
   orderPositions(ps, d);
-  a.n0 = (unsigned)d[0].n; a.n1 = (unsigned)d[1].n;
-  a.xs0 = d[0].xs; a.xs1 = d[1].xs; a.xs2 = d[2].xs;
-  a.zs0 = d[0].zs; a.zs1 = d[1].zs; a.zs2 = d[2].zs;
+  a.n0 = posDiv((unsigned)d[0].n); a.n1 = posDiv((unsigned)d[1].n);
+  unsigned* const strides[3][2] = {{&a.xs0, &a.zs0}, {&a.xs1, &a.zs1}, {&a.xs2, &a.zs2}};
+  for (int i = 0; i < 3; i++) {
+    if (d[i].n == 1) d[i].xs = d[i].zs = 0;                    // never multiplied
+    if (d[i].xs < 0 || d[i].zs < 0 || d[i].xs >> 32 != 0 || d[i].zs >> 32 != 0) return fastKronKernelNotFound;
+    *strides[i][0] = (unsigned)d[i].xs;
+    *strides[i][1] = (unsigned)d[i].zs;
+  }
   a.total = (unsigned)total;
   a.numTiles = (unsigned)((total + kSplitRows - 1) / kSplitRows);
   const bool al = ((uintptr_t)a.X & 15) == 0;
@@ -600,6 +697,11 @@ fastKronError launchGemmSplit(const Pass& ps, const LaunchCtx& cx) {
 
   a.vecZ = a.outT && a.Q % 4 == 0 && ((uintptr_t)a.Z & 15) == 0 && ((uintptr_t)a.Y & 15) == 0 && (d[0].n == 1 || m4(a.zs0)) &&
            (d[1].n == 1 || m4(a.zs1)) && (d[2].n == 1 || m4(a.zs2));
+  a.slotCols = a.N > 32 ? kBlockN : 32;
+  // A second accumulator for the small terms where there is room for at least four of h*h.
+  const unsigned ks = (a.P + 15) / 16, fit = (512 - aBuffers(ks) * 24 * ks) / a.slotCols;
+  a.slots = fit < kMaxSlots ? fit : kMaxSlots;
+  a.sSlots = a.slots >= 6 ? 2 : 1;
   const size_t factor = 3 * (size_t)((a.P + 63) / 64) * a.N * 128;
   const size_t stage = kSplitConvWarps * (size_t)kSplitStageElems * sizeof(float);    // one stage of every converter warp
   const size_t n = (kSplitSmem - 1024 - factor - (a.outT ? kXposeBytes : 0)) / stage;

@@ -3,8 +3,8 @@ sizes where they can go wrong: partial tiles, remainders of 16 and 32, both orie
 16-byte aligned, beta*Y in place of the result, values that a bf16 split cannot hold.
 
 Bound.  One step of P products in precision u errs by at most (P + 2) u of the sum of the products' magnitudes
-(one rounding per product for an FMA chain; for the split pass one accumulator rounding, of at most 2 u, per 16
-products of each of its six terms, and 2^-26 for the terms it leaves out).  Over the steps the bounds add up, and
+(one rounding per product for an FMA chain; for the split pass 2.5 u for each 16 products of h*h, a 32nd of that for each of the
+seven small terms, one rounding per accumulator and 2^-30 for l*l: test_split_precision.py has the tight checks).  Over the steps the bounds add up, and
 alpha and beta*Y add two roundings: |error| <= u * (sum (P_i + 4) + 4) * (|alpha| |X| |F| + |beta| |Y|)."""
 import ctypes
 import os
