@@ -12,6 +12,8 @@ constexpr unsigned kChainMaxQB = 8;                 // outputs of one column a t
 constexpr size_t kChainSmem3 = 74 * 1024;           // three CTAs per SM
 constexpr size_t kChainSmem2 = 112 * 1024;          // two
 constexpr size_t kChainSmemMax = kChainSmem2;
+// Resident CTAs of a tile of `smem` bytes: an SM has 228 KB, of which each takes 1 KB besides its own.
+inline unsigned chainCtasPerSm(size_t smem) { const size_t n = 228 * 1024 / (smem + 1024); return n > 3 ? 3 : (unsigned)n; }
 
 struct ChainShape {
   unsigned G, H;                                    // products of the P's and of the Q's

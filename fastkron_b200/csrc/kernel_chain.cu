@@ -341,9 +341,7 @@ static fastKronError launchChainT(const Pass& ps, const LaunchCtx& cx) {
     if (e != cudaSuccess) return cudaToFk(e);
     attr = true;
   }
-  unsigned perSm = (unsigned)(224 * 1024 / (s.smem + 1024));
-  if (perSm > 3) perSm = 3;
-  unsigned grid = (unsigned)cx.smCount * perSm;
+  unsigned grid = (unsigned)cx.smCount * chainCtasPerSm(s.smem);
   if (grid > a.numTiles) grid = a.numTiles;
   kern<<<grid, kChainThreads, s.smem, cx.stream>>>(a);
   return cudaToFk(cudaGetLastError());

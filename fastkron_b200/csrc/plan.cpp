@@ -302,7 +302,7 @@ static double groupCost(const Problem& pr, int f0, int f1) {
   // short runs of a strided side cost sectors
   double runs = 1;
   if (ps.xsG != 1 || ps.zsG != 1) { const double run = s.W * es; runs = run >= 64 ? 1 : run >= 32 ? 1.3 : 1.8; }
-  const double waves = std::ceil(pos / s.W) / (148.0 * (s.smem > kChainSmem3 ? 2 : 3));
+  const double waves = std::ceil(pos / s.W) / (148.0 * chainCtasPerSm(s.smem));
   return 4 + std::max(bytes / 5.0e6 * runs, macs / (f32 ? 7.5e6 : 3.2e6)) * (waves > 1 ? std::ceil(waves) / waves : 1);
 }
 

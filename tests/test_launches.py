@@ -102,3 +102,36 @@ def test_regrouping_honours_options(L):
         a = launches(L, "mkm", "f32", 8, [12] * 3, [12] * 3, **kw)
         b = launches(L, "mkm", "f32", 8, [12] * 3, [12] * 3, name="fkbDescribePlan", **kw)
         assert a == b and len(a) == 3
+
+
+def test_chain_tiles_get_the_ctas_per_sm_they_were_sized_for(tmp_path):
+    """Every group that chainShape accepts: the launcher's grid has the CTAs per SM that the tile was sized for (three
+    up to kChainSmem3, else two), and they fit."""
+    import os
+    import subprocess
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    src = tmp_path / "t.cpp"
+    src.write_text(r'''
+#include "chain_table.h"
+#include <stdio.h>
+using namespace fkb;
+int main() {
+  unsigned groups = 0, bad = 0;
+  for (int d = 0; d < 2; d++)
+    for (uint32_t p0 = 1; p0 <= 32; p0++) for (uint32_t q0 = 1; q0 <= 32; q0 += 3)
+      for (uint32_t p1 = 2; p1 <= 32; p1 += 1) for (uint32_t q1 = 2; q1 <= 32; q1 += 5)
+        for (uint32_t p2 = 1; p2 <= 16; p2 += 7) {
+          const uint32_t P[3] = {p0, p1, p2}, Q[3] = {q0, q1, p2};
+          ChainShape s;
+          if (!chainShape(d ? DType::F64 : DType::F32, p2 > 1 ? 3 : 2, P, Q, (p0 & 1) != 0, 1 << 20, &s)) continue;
+          groups++;
+          const unsigned n = chainCtasPerSm(s.smem);
+          if (s.smem > kChainSmemMax || n < (s.smem <= kChainSmem3 ? 3u : 2u) || n * (s.smem + 1024) > 228 * 1024) bad++;
+        }
+  printf("%u %u\n", groups, bad);
+}
+''')
+    exe = str(tmp_path / "t")
+    subprocess.check_call(["g++", "-O1", "-std=c++17", "-I", os.path.join(root, "include"), "-I", os.path.join(root, "fastkron_b200", "csrc"), str(src), "-o", exe])
+    groups, bad = map(int, subprocess.check_output([exe]).split())
+    assert groups > 10000 and bad == 0, (groups, bad)
