@@ -25,7 +25,7 @@ struct ChainShape {
 
 // False when the group does not fit shared memory.  `contig`: the group index is contiguous on the input or
 // the output side (columns are then written and read across the tile's rows, which wants an odd pitch).
-inline bool chainShape(DType dt, int nf, const uint32_t* P, const uint32_t* Q, bool contig, uint64_t total, ChainShape* s) {
+inline bool chainShape(DType dt, int nf, const uint32_t* P, const uint32_t* Q, bool contig, uint64_t total, int smCount, ChainShape* s) {
   const size_t es = dtypeSize(dt);
   const unsigned vec = (unsigned)(16 / es);
   uint64_t cur = 1, most[2], h = 1;
@@ -58,7 +58,7 @@ inline bool chainShape(DType dt, int nf, const uint32_t* P, const uint32_t* Q, b
   for (unsigned w = 16 * vec; w >= vec && !W; w /= 2) if (size(w) <= kChainSmem2) W = w;
   if (!W) return false;
   // narrower while the grid would leave SMs idle
-  while (W > vec && (total + W - 1) / W < 2 * 148) W /= 2;
+  while (W > vec && (total + W - 1) / W < 2 * (uint64_t)smCount) W /= 2;
   size(W);
   return true;
 }

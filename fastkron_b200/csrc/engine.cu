@@ -141,6 +141,7 @@ fastKronError Engine::run(Problem pr, const CallOperands& ops) {
   PlanOptions po;
   po.fusion = (options_ & fastKronOptionsUseFusion) != 0;
   po.haveT2 = ops.temp2 != nullptr;
+  po.smCount = smCount();
   int al = 16;
   auto upd = [&](const void* p) { int a = ptrAlign(p); if (a < al) al = a; };
   upd(ops.X); upd(ops.Z); upd(ops.temp1); upd(ops.temp2);

@@ -99,6 +99,7 @@ struct PlanOptions {
   size_t smemBudget = 200 * 1024;
   // pointer alignment of X / Z / temps in bytes (vector kernels need 16)
   int  align = 16;
+  int  smCount = 148;           // of the device the plan is for
 };
 
 // Build the list of passes for a problem.  Pure host code.

@@ -296,7 +296,7 @@ static fastKronError launchChainT(const Pass& ps, const LaunchCtx& cx) {
   ChainShape s;
   if (total == 0) return fastKronSuccess;
   if (total >= (1ull << 31) || cx.scatter.parts > 0 || cx.pSplit != 0 ||
-      !chainShape(cx.dt, ps.nf, ps.P, ps.Q, ps.xsG == 1 || ps.zsG == 1, total * cx.batch, &s))
+      !chainShape(cx.dt, ps.nf, ps.P, ps.Q, ps.xsG == 1 || ps.zsG == 1, total * cx.batch, cx.smCount, &s))
     return fastKronKernelNotFound;
   ChainArgs<T> a;
   a.X = (const T*)cx.src; a.Z = (T*)cx.dst; a.Y = (const T*)cx.Y;

@@ -284,7 +284,7 @@ static Pass groupPass(const Problem& pr, int f0, int f1) {
 // less by what a factor leaves of its tile (64, 32 or 16 wide, chunks of 32 or 16); a chain 5.0 TB/s and 7.5e12 or 3.2e12, in
 // whole waves of CTAs.  (Two of 31x31x31 fp64 in one launch: 66 us against 23 + 23, which the bytes alone do not say;
 // three of 12x12 fp32: 100 us against 87 + 61 + 55.)
-static double groupCost(const Problem& pr, int f0, int f1) {
+static double groupCost(const Problem& pr, const PlanOptions& opt, int f0, int f1) {
   const Pass ps = groupPass(pr, f0, f1);
   const bool f32 = pr.dt == DType::F32;
   const double es = (double)dtypeSize(pr.dt), pos = (double)ps.M * ps.A * ps.B;
@@ -298,11 +298,11 @@ static double groupCost(const Problem& pr, int f0, int f1) {
     return 4 + std::max(bytes / 3.0e6, macs / ((f32 ? 13e6 : 3.9e6) * fill));
   }
   ChainShape s;
-  if (!chainShape(pr.dt, ps.nf, ps.P, ps.Q, ps.xsG == 1 || ps.zsG == 1, (uint64_t)pos, &s)) return -1;
+  if (!chainShape(pr.dt, ps.nf, ps.P, ps.Q, ps.xsG == 1 || ps.zsG == 1, (uint64_t)pos, opt.smCount, &s)) return -1;
   // short runs of a strided side cost sectors
   double runs = 1;
   if (ps.xsG != 1 || ps.zsG != 1) { const double run = s.W * es; runs = run >= 64 ? 1 : run >= 32 ? 1.3 : 1.8; }
-  const double waves = std::ceil(pos / s.W) / (148.0 * chainCtasPerSm(s.smem));
+  const double waves = std::ceil(pos / s.W) / ((double)opt.smCount * chainCtasPerSm(s.smem));
   return 4 + std::max(bytes / 5.0e6 * runs, macs / (f32 ? 7.5e6 : 3.2e6)) * (waves > 1 ? std::ceil(waves) / waves : 1);
 }
 
@@ -325,7 +325,7 @@ void fuseLaunches(const Problem& pr, const PlanOptions& opt, Plan* plan) {
     best[0] = 0;
     for (int c = 1; c <= n; c++)
       for (int g = 1; g <= most && g <= c; g++) {
-        const double t = groupCost(pr, in[k + c - 1].f0, in[k + c - g].f0);
+        const double t = groupCost(pr, opt, in[k + c - 1].f0, in[k + c - g].f0);
         if (t >= 0 && best[c - g] + t < best[c]) { best[c] = best[c - g] + t; from[c] = c - g; }
       }
     if (best[n] >= 1e30) { out.insert(out.end(), in.begin() + k, in.begin() + e); k = e; continue; }

@@ -123,7 +123,7 @@ int main() {
         for (uint32_t p2 = 1; p2 <= 16; p2 += 7) {
           const uint32_t P[3] = {p0, p1, p2}, Q[3] = {q0, q1, p2};
           ChainShape s;
-          if (!chainShape(d ? DType::F64 : DType::F32, p2 > 1 ? 3 : 2, P, Q, (p0 & 1) != 0, 1 << 20, &s)) continue;
+          if (!chainShape(d ? DType::F64 : DType::F32, p2 > 1 ? 3 : 2, P, Q, (p0 & 1) != 0, 1 << 20, 148, &s)) continue;
           groups++;
           const unsigned n = chainCtasPerSm(s.smem);
           if (s.smem > kChainSmemMax || n < (s.smem <= kChainSmem3 ? 3u : 2u) || n * (s.smem + 1024) > 228 * 1024) bad++;
