@@ -42,7 +42,8 @@
 // Operands a bf16 split cannot hold are found while splitting: elements with a remainder after the third piece
 // (infinities, NaN, and numbers below about 2^-110 whose last bits lie under the smallest bf16 denormal 2^-133; the
 // tensor cores take and give denormals in full), and magnitudes from 2^127 or whose sums could overflow.  A row with such
-// an element, or every row when the factor has one, is recomputed by its epilogue thread as the plain FMA chain over p.
+// an element, or every row when the factor has one, takes the FMA chain over p instead, the numbers of the FMA kernels: the
+// epilogue leaves it out and marks the tile, and after the last tile the whole CTA contracts the marked ones from shared memory.
 #include <stdlib.h>
 
 #include <cuda_bf16.h>
@@ -66,6 +67,11 @@ constexpr int kSplitSmem = (227 - 3) * 1024;         // dynamic shared memory; t
 constexpr int kXposePitch = 36;                    // 32 columns and an odd number of 16-byte units per row
 constexpr size_t kXposeBytes = kSplitEpiWarps * 32 * kXposePitch * sizeof(float);
 constexpr unsigned kBlockN = 64;                   // columns of an accumulator: wider results go in blocks of 64
+constexpr unsigned kTileBits = 2048;               // marks of tiles with rows for the FMA chain; tiles that share one are looked at
+constexpr unsigned kFmaChunk = 16, kFmaPitch = kSplitRows + 4;   // p per stage of the FMA chain, elements between them
+constexpr unsigned kOutPitch = kBlockN + 4;        // elements between the rows of its result
+constexpr unsigned kFmaThreads = 512, kLoadX = kFmaChunk * kSplitRows / kFmaThreads, kLoadF = kFmaChunk * kBlockN / kFmaThreads;
+static_assert(kFmaChunk * (kFmaPitch + kBlockN) <= kSplitRows * kOutPitch && kFmaThreads <= kSplitThreads, "the result takes the place of a stage");
 // Steps of 16 products of h*h that share an accumulator.  With four, smooth one-signed factors (exp(-|i-j|/3)) err more than in
 // the FMA chain (3.7e-7 against 1.7e-7, 64x64 twice); with one the epilogue reads twice as many (64x64: 10.0 ms against 8.9).
 constexpr unsigned kHhSteps = 2;
@@ -169,10 +175,223 @@ __device__ __forceinline__ void split2(float x0, float x1, unsigned& h, unsigned
   left |= l0 | l1;
 }
 
+// Offset of position J by the strides s0, s1, s2 of its three indices.
+__device__ __forceinline__ long long positionOf(const SplitArgs& a, unsigned J, unsigned s0, unsigned s1, unsigned s2) {
+  const unsigned r0 = quot(J, a.n0), i0 = J - r0 * a.n0.d, i2 = quot(r0, a.n1), i1 = r0 - i2 * a.n1.d;
+  return (long long)((unsigned long long)i0 * s0 + (unsigned long long)i1 * s1 + (unsigned long long)i2 * s2);
+}
+
+// Columns c0 .. c0+31 of this lane's position J, whose results start at zoff, with alpha and beta*Y; executed by a whole
+// warp with scratch sc (32 rows of kXposePitch).
+__device__ __forceinline__ void storeBlock(const SplitArgs& a, float* sc, float (&r)[32], unsigned c0, unsigned J, long long zoff, bool store) {
+  const int lane = threadIdx.x & 31;
+  const bool epi = a.epilogue != 0;
+  const bool useY = epi && a.beta != 0.f && a.Y != nullptr;
+  const bool linear = a.n0.d == a.total;
+  if (!a.outT) {
+    float* z = a.Z + zoff + (long long)c0 * a.zsQ;
+    if (!epi) {
+      if (store && c0 + 32 <= a.Q) {
+#pragma unroll
+        for (unsigned i = 0; i < 32; i++, z += a.zsQ) *z = r[i];
+      } else if (store) {
+#pragma unroll
+        for (unsigned i = 0; i < 32; i++, z += a.zsQ)
+          if (c0 + i < a.Q) *z = r[i];
+      }
+    } else if (store) {
+      const float* y = a.Y + zoff + (long long)c0 * a.zsQ;
+#pragma unroll
+      for (unsigned g = 0; g < 32; g += 4) {            // Y may be Z: read a batch ahead of its stores
+        float yv[4];
+#pragma unroll
+        for (unsigned i = 0; i < 4; i++) yv[i] = useY && c0 + g + i < a.Q ? y[(long long)(g + i) * a.zsQ] : 0.f;
+#pragma unroll
+        for (unsigned i = 0; i < 4; i++, z += a.zsQ) {
+          float v = a.alpha * r[g + i];
+          if (useY) v = fmaf(a.beta, yv[i], v);
+          if (c0 + g + i < a.Q) *z = v;
+        }
+      }
+    }
+  } else {
+    // Lanes hold positions, the output wants lanes along q: through the warp's scratch, 32 columns (a whole
+    // 128-byte line of every row) at a time.
+    const unsigned stores = __ballot_sync(0xffffffffu, store);
+#pragma unroll
+    for (unsigned i = 0; i < 32; i += 4)
+      *reinterpret_cast<float4*>(sc + lane * kXposePitch + i) = make_float4(r[i], r[i + 1], r[i + 2], r[i + 3]);
+    __syncwarp();
+    // offset of row rr of this warp's 32, also on lanes whose own position lies beyond the last
+    auto rowOff = [&](unsigned rr) -> long long {
+      if (linear) return (long long)((unsigned long long)(J - (unsigned)lane + rr) * a.zs0);
+      return __shfl_sync(0xffffffffu, zoff, (int)rr);
+    };
+    // (reads of a batch of rows ahead of their stores: a store may alias the scratch as far as the compiler knows)
+    if (a.vecZ) {
+      const unsigned q = c0 + 4 * ((unsigned)lane & 7u);           // Q % 4 == 0: whole vectors
+#pragma unroll 1
+      for (unsigned b = 0; b < 32; b += 8) {
+        float4 v[2];
+        long long o[2];
+#pragma unroll
+        for (unsigned i = 0; i < 2; i++) {
+          const unsigned rr = b + 4 * i + ((unsigned)lane >> 3);
+          v[i] = *reinterpret_cast<const float4*>(sc + rr * kXposePitch + 4 * (lane & 7));
+          o[i] = rowOff(rr) + q;
+        }
+#pragma unroll
+        for (unsigned i = 0; i < 2; i++) {
+          const unsigned rr = b + 4 * i + ((unsigned)lane >> 3);
+          if (q >= a.Q || !(stores >> rr & 1u)) continue;
+          if (epi) {
+            v[i].x = a.alpha * v[i].x; v[i].y = a.alpha * v[i].y; v[i].z = a.alpha * v[i].z; v[i].w = a.alpha * v[i].w;
+            if (useY) {
+              const float4 y = *reinterpret_cast<const float4*>(a.Y + o[i]);
+              v[i].x = fmaf(a.beta, y.x, v[i].x); v[i].y = fmaf(a.beta, y.y, v[i].y);
+              v[i].z = fmaf(a.beta, y.z, v[i].z); v[i].w = fmaf(a.beta, y.w, v[i].w);
+            }
+          }
+          *reinterpret_cast<float4*>(a.Z + o[i]) = v[i];
+        }
+      }
+    } else {
+      const unsigned q = c0 + (unsigned)lane;
+#pragma unroll 2
+      for (unsigned b = 0; b < 32; b += 4) {
+        float v[4];
+#pragma unroll
+        for (unsigned i = 0; i < 4; i++) v[i] = sc[(b + i) * kXposePitch + lane];
+#pragma unroll
+        for (unsigned i = 0; i < 4; i++) {
+          const long long o = rowOff(b + i) + q;
+          if (q < a.Q && (stores >> (b + i) & 1u)) {
+            if (epi) { v[i] = a.alpha * v[i]; if (useY) v[i] = fmaf(a.beta, a.Y[o], v[i]); }
+            a.Z[o] = v[i];
+          }
+        }
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// Rows whose operands a split does not hold, after the tiles on the tensor cores: the FMA chain over p, by the whole CTA.  Stages
+// of kFmaChunk p go through registers into shared memory (past the L1, of which next to nothing is left) while 16 warps
+// contract the one before, 4 positions x 4 columns a thread.  A function of its own, so that it takes no registers from the
+// roles; what its loops need of the arguments is read once (through a reference each reading goes to memory).
+// marks == nullptr: every row.  268 MB in and out, a factor that cannot be split: 64x64 733 us (FMA kernel 190), 128x128 with 134 MB 1085
+// (338), 36x36 997 (680); a row in a thousand 264 / 429 / 374.  Bound by the latency of its stages: it is the route for rare operands.
+template <bool XT>
+__device__ __noinline__ void fmaTiles(const SplitArgs& args, float* xpose, float* ring, const unsigned* marks, unsigned rowHuge) {
+  const unsigned tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const unsigned first = blockIdx.x, step = gridDim.x;
+  const unsigned P = args.P, Q = args.Q, N = args.N, total = args.total;
+  const unsigned tiles = first < args.numTiles ? (args.numTiles - first + step - 1) / step : 0;
+  const float* const X = args.X;
+  const float* const F = args.F;
+  const long long xsP = args.xsP;
+  const bool fRows = args.fsQ == 1;                              // factor stored as [p][q], else [q][p]
+  // shared memory: [kFmaChunk][kFmaPitch] of X, [kFmaChunk][kBlockN] of the factor; the result takes their place
+  const unsigned xs = smemAddr(ring), fs = xs + kFmaChunk * kFmaPitch * 4u;
+  long long* const xo = reinterpret_cast<long long*>(ring + kSplitRows * kOutPitch);   // [kSplitRows], -1 beyond the last position
+  for (unsigned it = 0; it < tiles; it++) {
+    if (marks != nullptr && (marks[it % kTileBits / 32] >> (it & 31u) & 1u) == 0) continue;
+    const unsigned J0 = (first + it * step) * (unsigned)kSplitRows;
+    __syncthreads();
+    if (tid < kSplitRows) xo[tid] = J0 + tid < total ? positionOf(args, J0 + tid, args.xs0, args.xs1, args.xs2) : -1;
+    __syncthreads();
+    float vx[kLoadX], vf[kLoadF];
+    auto fetch = [&](unsigned p0, unsigned cb) {
+#pragma unroll
+      for (unsigned i = 0; i < kLoadX; i++) {
+        const unsigned e = i * kFmaThreads + tid, p = p0 + (XT ? e % kFmaChunk : e / kSplitRows);
+        const long long o = xo[XT ? e / kFmaChunk : e % kSplitRows];
+        vx[i] = o >= 0 && p < P ? __ldcg(X + o + p * xsP) : 0.f;
+      }
+#pragma unroll
+      for (unsigned i = 0; i < kLoadF; i++) {
+        const unsigned e = i * kFmaThreads + tid, p = p0 + (fRows ? e / kBlockN : e % kFmaChunk), q = cb + (fRows ? e % kBlockN : e / kFmaChunk);
+        vf[i] = p < P && q < Q ? __ldcg(F + (fRows ? p * Q + q : q * P + p)) : 0.f;
+      }
+    };
+    for (unsigned cb = 0; cb < N; cb += kBlockN) {
+      float r[16], mx = 0.f;
+      unsigned left = 0;
+#pragma unroll
+      for (unsigned i = 0; i < 16; i++) r[i] = 0.f;
+      if (tid < kFmaThreads) fetch(0, cb);
+#pragma unroll 1
+      for (unsigned p0 = 0; p0 < P; p0 += kFmaChunk) {
+        if (tid < kFmaThreads) {
+#pragma unroll
+          for (unsigned i = 0; i < kLoadX; i++) {
+            const unsigned e = i * kFmaThreads + tid;
+            ring[(XT ? e % kFmaChunk : e / kSplitRows) * kFmaPitch + (XT ? e / kFmaChunk : e % kSplitRows)] = vx[i];
+          }
+#pragma unroll
+          for (unsigned i = 0; i < kLoadF; i++) {
+            const unsigned e = i * kFmaThreads + tid;
+            ring[kFmaChunk * kFmaPitch + (fRows ? e : e % kFmaChunk * kBlockN + e / kFmaChunk)] = vf[i];
+          }
+        }
+        __syncthreads();
+        if (tid < kFmaThreads) {
+          if (p0 + kFmaChunk < P) fetch(p0 + kFmaChunk, cb);
+          unsigned x = xs + 16 * lane, f = fs + 16 * warp;
+          const unsigned n = min(P - p0, kFmaChunk);
+#pragma unroll 4
+          for (unsigned p = 0; p < n; p++, x += kFmaPitch * 4, f += kBlockN * 4) {
+            const float4 xv = ldShared4(x), fv = ldShared4(f);
+            const float xa[4] = {xv.x, xv.y, xv.z, xv.w};
+#pragma unroll
+            for (unsigned i = 0; i < 4; i++) {
+              r[4 * i] = fmaf(xa[i], fv.x, r[4 * i]);
+              r[4 * i + 1] = fmaf(xa[i], fv.y, r[4 * i + 1]);
+              r[4 * i + 2] = fmaf(xa[i], fv.z, r[4 * i + 2]);
+              r[4 * i + 3] = fmaf(xa[i], fv.w, r[4 * i + 3]);
+            }
+          }
+        }
+        if (marks != nullptr && warp < kSplitEpiWarps) {        // the converters' verdict on this thread's row
+#pragma unroll 2
+          for (unsigned p = 0; p < kFmaChunk; p += 2) {
+            const unsigned y = xs + (p * kFmaPitch + (warp & 3u) * 32u + lane) * 4u;
+            const float x0 = ldShared(y), x1 = ldShared(y + kFmaPitch * 4);
+            unsigned h, m, l;
+            split2(x0, x1, h, m, l, left);
+            mx = fmaxf(mx, fmaxf(fabsf(x0), fabsf(x1)));
+          }
+        }
+        __syncthreads();
+      }
+      // one position and 32 columns a thread, as the stores want them
+      if (tid < kFmaThreads) {
+#pragma unroll
+        for (unsigned i = 0; i < 4; i++)
+          *reinterpret_cast<float4*>(ring + (4 * lane + i) * kOutPitch + 4 * warp) = make_float4(r[4 * i], r[4 * i + 1], r[4 * i + 2], r[4 * i + 3]);
+      }
+      __syncthreads();
+      if (warp < kSplitEpiWarps) {
+        const unsigned row = (warp & 3u) * 32u + lane, c0 = (warp >> 2) * 32u, J = J0 + row;
+        float z[32];
+#pragma unroll
+        for (unsigned i = 0; i < 32; i += 4) {
+          const float4 v = ldShared4(xs + (row * kOutPitch + c0 + i) * 4u);
+          z[i] = v.x; z[i + 1] = v.y; z[i + 2] = v.z; z[i + 3] = v.w;
+        }
+        const bool mine = marks == nullptr || (left & 0xFFFFu) != 0 || __float_as_uint(mx) >= rowHuge;
+        storeBlock(args, xpose + warp * 32 * kXposePitch, z, cb + c0, J, positionOf(args, J, args.zs0, args.zs1, args.zs2), J < total && mine);
+      }
+      __syncthreads();
+    }
+  }
+}
+
 // XT: the contracted index is contiguous in X (lanes load along p); otherwise lanes load along j.
 // KS: steps of 16 along the contraction.
 template <bool XT, int KS>
-__global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitArgs a) {
+__global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const __grid_constant__ SplitArgs a) {
   constexpr unsigned K = 16 * KS, ks = KS, half = K / 2;     // half: TMEM columns of one piece of A
   constexpr unsigned slabs = (K + 63) / 64;
   constexpr unsigned hSlots = (KS + kHhSteps - 1) / kHhSteps;  // accumulators of h*h per block of columns
@@ -186,6 +405,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   __shared__ unsigned tmemBaseSlot;
   __shared__ int abortFlag, factorSpecial;
   __shared__ unsigned rowHuge;
+  __shared__ unsigned tileMarks[kTileBits / 32], anyMark;
   __shared__ unsigned factorMax;                             // float bits of the largest magnitude
   __shared__ unsigned short rowState[8][kSplitRows];  // tile it, position: (it >> 3) + 1 if its row cannot be split
 
@@ -198,7 +418,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     // dFull: the commit of the MMAs, and an ordinary arrival that carries what the converters wrote (rowState)
     for (unsigned i = 0; i < kMaxSlots; i++) { mbarInit(&dFull[i], 2); mbarInit(&dEmpty[i], kSplitEpiWarps); }
     mbarInit(&drained, 1);
-    abortFlag = 0; factorSpecial = 0;
+    abortFlag = 0; factorSpecial = 0; anyMark = 0;
     factorMax = 0;
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -207,6 +427,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;\n" ::: "memory");
   }
   __syncthreads();
+  for (unsigned i = tid; i < kTileBits / 32; i += kSplitThreads) tileMarks[i] = 0;
   for (unsigned i = tid; i < 8 * kSplitRows; i += kSplitThreads) (&rowState[0][0])[i] = 0;
   // factor -> three bf16 copies, row q, k contiguous: 16-byte unit (k % 64) / 8 XOR (q % 8)
   unsigned fMax = 0, fLeft = 0;
@@ -246,16 +467,12 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
   const unsigned dCol = tmemBase + nA * aCols;
 
   const unsigned first = blockIdx.x, step = gridDim.x;
-  const unsigned myTiles = first < a.numTiles ? (a.numTiles - first + step - 1) / step : 0;
+  const unsigned myTiles = first < a.numTiles && factorSpecial == 0 ? (a.numTiles - first + step - 1) / step : 0;
 
   if (warp < kSplitEpiWarps) {
     // ---- epilogue ----------------------------------------------------------------------------
     const unsigned quarter = (unsigned)warp & 3u, part = (unsigned)warp >> 2;
-    const bool epi = a.epilogue != 0;
-    const bool useY = epi && a.beta != 0.f && a.Y != nullptr;
-    const bool allSpecial = factorSpecial != 0;
-    const bool linear = a.n0.d == a.total;
-    float* sc = xpose + warp * 32 * kXposePitch;
+    float* const sc = xpose + warp * 32 * kXposePitch;
     // take(): the MMAs into accumulator `sl` are complete; give(): this warp has read it.  Each set has full-barriers of
     // its own (a wait for a later phase than the next is none); bit `sl` of phases: parity of the next one of `sl`.
     unsigned sSlot = 0, slot = a.sSlots, phases = 0;
@@ -274,8 +491,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     for (unsigned it = 0; alive && it < myTiles; it++) {
       const unsigned J = (first + it * step) * (unsigned)kSplitRows + quarter * 32u + (unsigned)lane;
       const bool live = J < a.total;
-      const unsigned r0 = quot(J, a.n0), i0 = J - r0 * a.n0.d, i2 = quot(r0, a.n1), i1 = r0 - i2 * a.n1.d;
-      const long long zoff = (long long)((unsigned long long)i0 * a.zs0 + (unsigned long long)i1 * a.zs1 + (unsigned long long)i2 * a.zs2);
+      const long long zoff = positionOf(a, J, a.zs0, a.zs1, a.zs2);
       bool special = false, store = false;
 #pragma unroll 1
       for (unsigned cb = 0; cb < a.N; cb += kBlockN) {
@@ -305,108 +521,17 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
         }
         if (!alive || !take(sSlot)) { alive = false; break; }
         if (cb == 0) {
-          special = live && (allSpecial || rowState[it & 7][quarter * 32 + lane] == (unsigned short)((it >> 3) + 1u));
+          special = live && rowState[it & 7][quarter * 32 + lane] == (unsigned short)((it >> 3) + 1u);
           store = live && !special;
         }
         if (c0 < a.N) addFrom(sSlot);
         give(sSlot);
         if (++sSlot == a.sSlots) sSlot = 0;
-        if (!a.outT) {
-          float* z = a.Z + zoff + (long long)c0 * a.zsQ;
-          if (!epi) {
-            if (store && c0 + 32 <= a.Q) {
-#pragma unroll
-              for (unsigned i = 0; i < 32; i++, z += a.zsQ) *z = r[i];
-            } else if (store) {
-#pragma unroll
-              for (unsigned i = 0; i < 32; i++, z += a.zsQ)
-                if (c0 + i < a.Q) *z = r[i];
-            }
-          } else if (store) {
-            const float* y = a.Y + zoff + (long long)c0 * a.zsQ;
-#pragma unroll
-            for (unsigned g = 0; g < 32; g += 4) {            // Y may be Z: read a batch ahead of its stores
-              float yv[4];
-#pragma unroll
-              for (unsigned i = 0; i < 4; i++) yv[i] = useY && c0 + g + i < a.Q ? y[(long long)(g + i) * a.zsQ] : 0.f;
-#pragma unroll
-              for (unsigned i = 0; i < 4; i++, z += a.zsQ) {
-                float v = a.alpha * r[g + i];
-                if (useY) v = fmaf(a.beta, yv[i], v);
-                if (c0 + g + i < a.Q) *z = v;
-              }
-            }
-          }
-        } else {
-          // Lanes hold positions, the output wants lanes along q: through the warp's scratch, 32 columns (a whole
-          // 128-byte line of every row) at a time.
-          const unsigned stores = __ballot_sync(0xffffffffu, store);
-#pragma unroll
-          for (unsigned i = 0; i < 32; i += 4)
-            *reinterpret_cast<float4*>(sc + lane * kXposePitch + i) = make_float4(r[i], r[i + 1], r[i + 2], r[i + 3]);
-          __syncwarp();
-          // offset of row rr of this warp's 32, also on lanes whose own position lies beyond the last
-          auto rowOff = [&](unsigned rr) -> long long {
-            if (linear) return (long long)((unsigned long long)(J - (unsigned)lane + rr) * a.zs0);
-            return __shfl_sync(0xffffffffu, zoff, (int)rr);
-          };
-          // (reads of a batch of rows ahead of their stores: a store may alias the scratch as far as the compiler knows)
-          if (a.vecZ) {
-            const unsigned q = c0 + 4 * ((unsigned)lane & 7u);           // Q % 4 == 0: whole vectors
-#pragma unroll 1
-            for (unsigned b = 0; b < 32; b += 8) {
-              float4 v[2];
-              long long o[2];
-#pragma unroll
-              for (unsigned i = 0; i < 2; i++) {
-                const unsigned rr = b + 4 * i + ((unsigned)lane >> 3);
-                v[i] = *reinterpret_cast<const float4*>(sc + rr * kXposePitch + 4 * (lane & 7));
-                o[i] = rowOff(rr) + q;
-              }
-#pragma unroll
-              for (unsigned i = 0; i < 2; i++) {
-                const unsigned rr = b + 4 * i + ((unsigned)lane >> 3);
-                if (q >= a.Q || !(stores >> rr & 1u)) continue;
-                if (epi) {
-                  v[i].x = a.alpha * v[i].x; v[i].y = a.alpha * v[i].y; v[i].z = a.alpha * v[i].z; v[i].w = a.alpha * v[i].w;
-                  if (useY) {
-                    const float4 y = *reinterpret_cast<const float4*>(a.Y + o[i]);
-                    v[i].x = fmaf(a.beta, y.x, v[i].x); v[i].y = fmaf(a.beta, y.y, v[i].y);
-                    v[i].z = fmaf(a.beta, y.z, v[i].z); v[i].w = fmaf(a.beta, y.w, v[i].w);
-                  }
-                }
-                *reinterpret_cast<float4*>(a.Z + o[i]) = v[i];
-              }
-            }
-          } else {
-            const unsigned q = c0 + (unsigned)lane;
-#pragma unroll 2
-            for (unsigned b = 0; b < 32; b += 4) {
-              float v[4];
-#pragma unroll
-              for (unsigned i = 0; i < 4; i++) v[i] = sc[(b + i) * kXposePitch + lane];
-#pragma unroll
-              for (unsigned i = 0; i < 4; i++) {
-                const long long o = rowOff(b + i) + q;
-                if (q < a.Q && (stores >> (b + i) & 1u)) {
-                  if (epi) { v[i] = a.alpha * v[i]; if (useY) v[i] = fmaf(a.beta, a.Y[o], v[i]); }
-                  a.Z[o] = v[i];
-                }
-              }
-            }
-          }
-          __syncwarp();
-        }
+        storeBlock(a, sc, r, c0, J, zoff, store);
       }
-      if (alive && special && part == 0) {
-        const float* x = a.X + (unsigned long long)i0 * a.xs0 + (unsigned long long)i1 * a.xs1 + (unsigned long long)i2 * a.xs2;
-        for (unsigned q = 0; q < a.Q; q++) {
-          float acc = 0.f;
-          for (unsigned p = 0; p < a.P; p++) acc = fmaf(x[(long long)p * a.xsP], a.F[(long long)p * a.fsP + (long long)q * a.fsQ], acc);
-          const long long o = zoff + (long long)q * a.zsQ;
-          if (epi) { acc = a.alpha * acc; if (useY) acc = fmaf(a.beta, a.Y[o], acc); }
-          a.Z[o] = acc;
-        }
+      if (part == 0 && __any_sync(0xffffffffu, special) && lane == 0) {
+        atomicOr(&tileMarks[it % kTileBits / 32], 1u << (it & 31u));
+        anyMark = 1;
       }
     }
   } else if (warp < kSplitMmaWarp) {
@@ -424,10 +549,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     // lane / 4 + 8 i, in units of 16 bytes.  ldMask: which of them exist.
     long long ldOff = 0;
     unsigned ldRow[XT ? 4 : 1];
-    auto offsetOf = [&](unsigned J) {
-      const unsigned r0 = quot(J, a.n0), i0 = J - r0 * a.n0.d, i2 = quot(r0, a.n1), i1 = r0 - i2 * a.n1.d;
-      return (long long)((unsigned long long)i0 * a.xs0 + (unsigned long long)i1 * a.xs1 + (unsigned long long)i2 * a.xs2);
-    };
+    auto offsetOf = [&](unsigned J) { return positionOf(a, J, a.xs0, a.xs1, a.xs2); };
     auto load = [&](unsigned st) {
       if (ldN < chunks) {
         const unsigned tile = ldN / ks;
@@ -619,6 +741,7 @@ __global__ void __launch_bounds__(kSplitThreads, 1) gemmSplitKernel(const SplitA
     fenceAfterSync();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmemBase), "r"(512) : "memory");
   }
+  if (abortFlag == 0 && (factorSpecial != 0 || anyMark != 0)) fmaTiles<XT>(a, xpose, ring, factorSpecial != 0 ? nullptr : tileMarks, rowHuge);
 }
 
 static unsigned long long gSplitLaunches = 0;

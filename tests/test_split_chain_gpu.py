@@ -28,6 +28,12 @@ def lib():
     assert L.fkbGemmSplitTimeouts() == 0
 
 
+@pytest.fixture(autouse=True)
+def split_on(lib):
+    yield
+    lib.fkbSetSplitOff(0)           # process-wide: also after a test that failed while it was set
+
+
 def product(x, fs):
     t = x
     for f in reversed(fs):
@@ -202,6 +208,47 @@ def test_split_pass_keeps_small_elements_beside_large_ones(lib, small_in):
     xn, fn = x.astype(np.float64), f.astype(np.float64)
     err, mag = np.abs(z - xn @ fn), np.abs(xn) @ np.abs(fn)
     assert np.all(err <= 2.0 ** -24 * (P + 8) * mag + P * 2.0 ** -149), np.max(err / np.maximum(mag, 1e-300))
+
+
+@pytest.mark.parametrize("where", ["factor", "every row", "some rows", "one row"])
+@pytest.mark.parametrize("mm,tx,tf,beta,M,P,Q", [("mkm", 0, 0, 1.0, 40000, 64, 48), ("kmm", 0, 1, 0.0, 30001, 33, 70), ("kmm", 1, 0, 0.5, 20000, 127, 128),
+                                                 ("mkm", 1, 0, 0.0, 25000, 128, 127)])
+def test_split_pass_contracts_what_it_cannot_split_like_the_fma_kernels(lib, where, mm, tx, tf, beta, M, P, Q):
+    """Rows with elements that a split does not hold, and every row when the factor has one, are the FMA chain's to the
+    last bit, in several tiles per CTA, with partial tiles, both layouts, and beta*Y in place of the result (Y is Z)."""
+    import torch
+    import fastkron_b200
+    g = torch.Generator(device="cuda").manual_seed(5)
+    x, f = torch.rand(M, P, device="cuda", generator=g) - 0.5, torch.rand(P, Q, device="cuda", generator=g) - 0.5
+    rows = {"factor": slice(None), "every row": slice(None), "some rows": slice(3, None, 331), "one row": slice(M - 1, M)}[where]
+    if where == "factor":
+        f[P - 1, Q - 1] = 1.2345e-39
+    else:
+        x[rows, P // 2] = 1.2345e-39
+        x[rows, P - 1] *= 1e-36
+    y = torch.rand(M, Q, device="cuda", generator=g)
+    xm, fm, ym = (x, f, y) if mm == "mkm" else (x.t(), f.t(), y.t())
+    xd = xm.t().contiguous().t() if tx else xm.contiguous()
+    fd = fm.t().contiguous().t() if tf else fm.contiguous()
+    h = fastkron_b200.FastKron()
+    opx, opf = (2 if tx else 1), (2 if tf else 1)
+    t = [torch.empty(M * max(P, Q), device="cuda") for _ in range(2)]
+
+    def run():
+        z = ym.contiguous().clone()
+        h.raw_gemm(mm, "s", M, [P], [Q], xd.data_ptr(), opx, [fd.data_ptr()], opf, z.data_ptr(), 2.0, beta, z.data_ptr() if beta else 0,
+                   t[0].data_ptr(), t[1].data_ptr())
+        return z if mm == "mkm" else z.t()
+    n0 = lib.fkbGemmSplitLaunches()
+    z = run()
+    assert lib.fkbGemmSplitLaunches() == n0 + 1
+    lib.fkbSetSplitOff(1)
+    w = run()
+    lib.fkbSetSplitOff(0)
+    h.close()
+    assert torch.equal(z[rows], w[rows])
+    d = lambda v: v.cpu().numpy().astype(np.float64)
+    check(d(z), d(x), [d(f)], 2.0, beta, d(y), 2.0 ** -24)
 
 
 CHAIN = [
