@@ -23,9 +23,11 @@ struct ChainShape {
   size_t offB, offF, offT, smem;                    // bytes: second buffer, factors, column tables, total
 };
 
-// False when the group does not fit shared memory.  `contig`: the group index is contiguous on the input or
+// False when the kernel does not take the group: its tile does not fit shared memory or the positions need more than 31
+// bits.  The planner forms no other groups, and the launcher declines no other (a group has no kernel to fall back to).  `contig`: the group index is contiguous on the input or
 // the output side (columns are then written and read across the tile's rows, which wants an odd pitch).
 inline bool chainShape(DType dt, int nf, const uint32_t* P, const uint32_t* Q, bool contig, uint64_t total, int smCount, ChainShape* s) {
+  if (total >= (1ull << 31)) return false;
   const size_t es = dtypeSize(dt);
   const unsigned vec = (unsigned)(16 / es);
   uint64_t cur = 1, most[2], h = 1;

@@ -40,12 +40,9 @@ struct ChainArgs {
   unsigned W, logW, pitch, offB, offF, offT;
   unsigned n0, n1;
   long long xs0, xs1, xs2, xsG, zs0, zs1, zs2, zsG;
-  unsigned total, tilesPerEntry, numTiles;
+  unsigned total, numTiles;
   int vecX, vecZ, epilogue;
   T alpha, beta;
-  unsigned batch;
-  int batchedF;
-  unsigned long long bsX, bsZ, bsY, bsF[kMaxGroup];
 };
 
 // acc[q][c] += f[q] * x[c]; fp32 with the packed FMA (two independent IEEE FMAs per instruction)
@@ -139,11 +136,11 @@ __global__ void __launch_bounds__(kChainThreads, 3) chainKernel(const __grid_con
   const unsigned logC = a.logW - (VEC == 4 ? 2 : 1);
 
   // factor k as [p][block][fb], blocks of qb outputs padded to whole vectors
-  auto loadFactors = [&](unsigned bt) {
+  {
     T* d = Fs;
     for (int k = 0; k < a.nf; k++) {
       const unsigned row = a.nb[k].d * a.fb[k];
-      const T* F = a.F[k] + bt * a.bsF[k];
+      const T* F = a.F[k];
       for (unsigned i = tid; i < a.P[k] * a.Q[k]; i += kChainThreads) {
         unsigned p, q;
         if (a.fsQ[k] == 1) { p = i / a.Q[k]; q = i - p * a.Q[k]; } else { q = i / a.P[k]; p = i - q * a.P[k]; }   // the stored order
@@ -152,15 +149,10 @@ __global__ void __launch_bounds__(kChainThreads, 3) chainKernel(const __grid_con
       }
       d += a.P[k] * row;
     }
-  };
-  loadFactors(0);
-  unsigned curEntry = 0;
+  }
 
-  for (unsigned t = blockIdx.x; t < a.numTiles; t += gridDim.x) {
-    unsigned bt = 0, tile = t;
-    if (a.batch > 1) { bt = t / a.tilesPerEntry; tile = t - bt * a.tilesPerEntry; }
+  for (unsigned tile = blockIdx.x; tile < a.numTiles; tile += gridDim.x) {
     __syncthreads();                                 // the previous tile has been stored
-    if (a.batchedF && bt != curEntry) { loadFactors(bt); curEntry = bt; }
     if (tid < a.W) {
       const unsigned J = tile * a.W + tid;
       const unsigned r0 = J / a.n0, i0 = J - r0 * a.n0, i2 = r0 / a.n1, i1 = r0 - i2 * a.n1;
@@ -171,7 +163,7 @@ __global__ void __launch_bounds__(kChainThreads, 3) chainKernel(const __grid_con
     __syncthreads();
 
     // ---- load --------------------------------------------------------------------------------
-    const T* X = a.X + bt * a.bsX;
+    const T* X = a.X;
     if (a.xsG == 1) {
       const unsigned units = a.G.d << logC;
 #pragma unroll 4
@@ -231,10 +223,10 @@ __global__ void __launch_bounds__(kChainThreads, 3) chainKernel(const __grid_con
     }
 
     // ---- store (alpha / beta*Y on the epilogue pass) -----------------------------------------------
-    T* Z = a.Z + bt * a.bsZ;
+    T* Z = a.Z;
     const bool epi = a.epilogue != 0;
     const bool useY = epi && a.beta != T(0) && a.Y != nullptr;
-    const T* Y = useY ? a.Y + bt * a.bsY : nullptr;
+    const T* Y = a.Y;
     if (a.zsG == 1) {
       const unsigned units = a.H.d << logC;
       for (unsigned u = tid; u < units; u += kChainThreads) {
@@ -295,21 +287,18 @@ static fastKronError launchChainT(const Pass& ps, const LaunchCtx& cx) {
   const uint64_t total = ps.M * ps.A * ps.B;
   ChainShape s;
   if (total == 0) return fastKronSuccess;
-  if (total >= (1ull << 31) || cx.scatter.parts > 0 || cx.pSplit != 0 ||
-      !chainShape(cx.dt, ps.nf, ps.P, ps.Q, ps.xsG == 1 || ps.zsG == 1, total * cx.batch, cx.smCount, &s))
+  if (cx.batch > 1 || cx.scatter.parts > 0 || cx.pSplit != 0 ||
+      !chainShape(cx.dt, ps.nf, ps.P, ps.Q, ps.xsG == 1 || ps.zsG == 1, total, cx.smCount, &s))
     return fastKronKernelNotFound;
   ChainArgs<T> a;
   a.X = (const T*)cx.src; a.Z = (T*)cx.dst; a.Y = (const T*)cx.Y;
   a.nf = ps.nf;
-  a.batch = cx.batch; a.bsX = cx.bsX; a.bsZ = cx.bsZ; a.bsY = cx.bsY; a.batchedF = 0;
   unsigned outer = 1, inner = 1;
   for (int k = 0; k < ps.nf; k++) {
     a.F[k] = (const T*)cx.F[k];
     a.P[k] = ps.P[k]; a.Q[k] = ps.Q[k]; a.qb[k] = s.qb[k]; a.fb[k] = s.fb[k]; a.nb[k] = fastDiv(s.nb[k]);
     // (p, q) of every factor lies as factor 0's stride pair says: one of the two is 1
     if (cx.fPMajor) { a.fsP[k] = ps.Q[k]; a.fsQ[k] = 1; } else { a.fsP[k] = 1; a.fsQ[k] = ps.P[k]; }
-    a.bsF[k] = cx.bsF[k];
-    if (cx.batch > 1 && cx.bsF[k] != 0) a.batchedF = 1;
     a.outer[k] = outer;
     outer *= ps.P[k];
   }
@@ -324,14 +313,11 @@ static fastKronError launchChainT(const Pass& ps, const LaunchCtx& cx) {
   a.xs0 = d[0].xs; a.xs1 = d[1].xs; a.xs2 = d[2].xs; a.xsG = ps.xsG;
   a.zs0 = d[0].zs; a.zs1 = d[1].zs; a.zs2 = d[2].zs; a.zsG = ps.zsG;
   auto al16 = [](const void* p) { return ((uintptr_t)p & 15) == 0; };
-  a.vecX = al16(a.X) && positionsVectorise(d, true, a.xsG, VEC) && (cx.batch == 1 || a.bsX % VEC == 0);
-  a.vecZ = al16(a.Z) && (a.Y == nullptr || al16(a.Y)) && positionsVectorise(d, false, a.zsG, VEC) &&
-           (cx.batch == 1 || (a.bsZ % VEC == 0 && a.bsY % VEC == 0));
+  a.vecX = al16(a.X) && positionsVectorise(d, true, a.xsG, VEC);
+  a.vecZ = al16(a.Z) && (a.Y == nullptr || al16(a.Y)) && positionsVectorise(d, false, a.zsG, VEC);
   a.alpha = (T)cx.alpha; a.beta = (T)cx.beta; a.epilogue = ps.epilogue ? 1 : 0;
   a.total = (unsigned)total;
-  a.tilesPerEntry = (a.total + a.W - 1) / a.W;
-  if ((uint64_t)a.tilesPerEntry * a.batch >= (1ull << 31)) return fastKronKernelNotFound;
-  a.numTiles = a.tilesPerEntry * a.batch;
+  a.numTiles = (a.total + a.W - 1) / a.W;
 
   auto kern = chainKernel<T>;
   static bool attrDev[kMaxDevices] = {false};

@@ -50,7 +50,7 @@ struct LaunchCtx {
 
 // True when the kernel that runs `ps` takes a strided batch in one launch.
 inline bool passBatchCapable(const Pass& ps) {
-  if (ps.kind == KernelKind::Generic || ps.kind == KernelKind::Chain) return true;
+  if (ps.kind == KernelKind::Generic) return true;
   if (ps.kind == KernelKind::Gemm) return ps.variant == 3;
   return ps.kind == KernelKind::Tile && ps.variant == 0;
 }

@@ -308,7 +308,7 @@ static double groupCost(const Problem& pr, const PlanOptions& opt, int f0, int f
 
 void fuseLaunches(const Problem& pr, const PlanOptions& opt, Plan* plan) {
   // strided batches and the forward variants keep one launch per pass
-  if (pr.batch > 1 || pr.forward || !opt.fusion || opt.forceGeneric || gForceGeneric || opt.isolateFirst) return;
+  if (pr.batch > 1 || pr.forward || !opt.fusion || opt.forceGeneric || gForceGeneric) return;
   int most = kMaxGroup;
   if (opt.maxFuse > 0 && opt.maxFuse < most) most = opt.maxFuse;
   if (gMaxFuseOverride > 0 && gMaxFuseOverride < most) most = gMaxFuseOverride;

@@ -135,3 +135,14 @@ int main() {
     subprocess.check_call(["g++", "-O1", "-std=c++17", "-I", os.path.join(root, "include"), "-I", os.path.join(root, "fastkron_b200", "csrc"), str(src), "-o", exe])
     groups, bad = map(int, subprocess.check_output([exe]).split())
     assert groups > 10000 and bad == 0, (groups, bad)
+
+
+def test_a_chain_group_has_one_admission_rule():
+    """A group of several factors has no kernel to fall back to, so the launcher may decline nothing that the planner forms:
+    besides chainShape, which both ask, only calls that never have groups (batches, redistribution over GPUs)."""
+    import os
+    src = open(os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "fastkron_b200", "csrc", "kernel_chain.cu")).read()
+    guards = re.findall(r"if \(([^;{}]*?)\)\s*return fastKronKernelNotFound;", src, re.S)
+    assert len(guards) == 1, guards
+    terms = {re.sub(r"\s+", " ", t).strip() for t in guards[0].split("||")} - {"ps.zsG == 1, total, cx.smCount, &s)"}
+    assert {t for t in terms if not t.startswith("!chainShape(")} == {"cx.batch > 1", "cx.scatter.parts > 0", "cx.pSplit != 0"}, terms
