@@ -40,8 +40,9 @@ inline bool gemmAnyEligible(uint32_t P, uint32_t Q) {
 // number of positions (rows of the contraction).  Measured on B200, FMA kernels -> this one, 25 million elements, pass
 // with p contiguous / with j contiguous: 36x36 182/158 -> 83/68 us, 64x64 85/84 -> 59/48, 100x100 229/207 -> 67/62; 48 -> 24 columns 51/27
 // -> 48/25, about even, and 64 -> 17 loses (55/21 -> 67/17: the fixed work per tile is spread over few outputs).  Below 24x24 the FMA
-// kernels are bound by memory themselves (24x24 three times, 256 rows: 58 us, 78 us here).  From 1024 positions (eight tiles)
-// on the launches take the same time (64x64: 12.4 and 13.7 us); fewer have never been faster here.
+// kernels are bound by memory themselves (24x24 three times, 256 rows: 58 us, 78 us here).  At 1024 positions (eight tiles) a
+// launch takes 12.4 us on the FMA kernel and 13.7 here (64x64); fewer have never been faster here.  (These times are the
+// six-product form's; the present one takes 1.05 to 1.3 times as long.  Between 24x24 and 36x36 the line is not measured.)
 inline bool gemmSplitEligible(uint32_t P, uint32_t Q, uint64_t total) {
   return P >= 17 && Q >= 20 && P <= 128 && Q <= 128 && P * Q >= 1024 && total >= 1024 && total < (1ull << 31);
 }
