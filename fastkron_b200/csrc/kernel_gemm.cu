@@ -96,34 +96,39 @@ static fastKronError launchGemmOne(const Pass& ps, const LaunchCtx& cx, int mode
 // and stays scalar.
 static fastKronError launchGemmFixed(const Pass& ps, const LaunchCtx& cx);
 
-// The split tensor-core kernel where its rule admits the pass, the fixed-shape FMA kernels where they
-// apply, the any-shape kernel otherwise.
+// What the fixed-shape kernels, TF32 ones among them, take.
+static bool fixedForm(const Pass& ps, const LaunchCtx& cx) {
+  if (ps.variant == 3 || ps.nf != 1 || ps.xsB != 1 || ps.zsB != 1) return false;
+  const uint32_t P = ps.P[0], Q = ps.Q[0];
+  if (!gemmEligible(cx.dt, P, Q, ps.B)) return false;
+  // dense [chunks][P][B] -> [chunks][Q][B] only
+  if (ps.xsG != (int64_t)ps.B || ps.zsG != (int64_t)ps.B || ps.xsA != (int64_t)(P * ps.B) || ps.zsA != (int64_t)(Q * ps.B)) return false;
+  if (ps.M > 1 && (ps.xsM != (int64_t)(ps.A * P * ps.B) || ps.zsM != (int64_t)(ps.A * Q * ps.B))) return false;
+  if (((uintptr_t)cx.src | (uintptr_t)cx.dst | (uintptr_t)cx.Y) & 15) return false;
+  return !(cx.fsQ == 1 && (((uintptr_t)cx.F[0]) & 15));
+}
+
+// The TF32 kernel where a handle asked for it and it takes the pass; then, whatever the handle's options, the split
+// tensor-core kernel where its rule admits the pass, the fixed-shape FMA kernels where they apply, the any-shape kernel
+// otherwise.
 fastKronError launchGemm(const Pass& ps, const LaunchCtx& cx) {
-  if (!cx.tf32) {
-    const fastKronError e = launchGemmSplit(ps, cx);
+  const bool fixed = fixedForm(ps, cx);
+  if (cx.tf32 && cx.dt == DType::F32 && fixed) {
+    const fastKronError e = launchGemmTf32(ps, cx);
     if (e != fastKronKernelNotFound) return e;
   }
-  if (ps.variant != 3) {
-    const fastKronError e = launchGemmFixed(ps, cx);
+  fastKronError e = launchGemmSplit(ps, cx);
+  if (e != fastKronKernelNotFound) return e;
+  if (fixed) {
+    e = launchGemmFixed(ps, cx);
     if (e != fastKronKernelNotFound) return e;
   }
   return launchGemmAny(ps, cx);
 }
 
 static fastKronError launchGemmFixed(const Pass& ps, const LaunchCtx& cx) {
-  if (ps.nf != 1 || ps.xsB != 1 || ps.zsB != 1) return fastKronKernelNotFound;
   const uint32_t P = ps.P[0], Q = ps.Q[0];
-  if (!gemmEligible(cx.dt, P, Q, ps.B)) return fastKronKernelNotFound;
-  // dense [chunks][P][B] -> [chunks][Q][B] only
-  if (ps.xsG != (int64_t)ps.B || ps.zsG != (int64_t)ps.B || ps.xsA != (int64_t)(P * ps.B) || ps.zsA != (int64_t)(Q * ps.B)) return fastKronKernelNotFound;
-  if (ps.M > 1 && (ps.xsM != (int64_t)(ps.A * P * ps.B) || ps.zsM != (int64_t)(ps.A * Q * ps.B))) return fastKronKernelNotFound;
-  if (((uintptr_t)cx.src | (uintptr_t)cx.dst | (uintptr_t)cx.Y) & 15) return fastKronKernelNotFound;
-  if (cx.fsQ == 1 && (((uintptr_t)cx.F[0]) & 15)) return fastKronKernelNotFound;
   const bool xt = ps.B == 1;
-  if (cx.tf32 && cx.dt == DType::F32) {
-    const fastKronError e = launchGemmTf32(ps, cx);
-    if (e != fastKronKernelNotFound) return e;          // shapes it does not take run in fp32 below
-  }
   if (cx.dt == DType::F32) {
     constexpr int TJ = 128;
     const int mode = xt ? 2 : (ps.B % TJ == 0 ? 0 : 1);

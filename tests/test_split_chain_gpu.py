@@ -251,6 +251,27 @@ def test_split_pass_contracts_what_it_cannot_split_like_the_fma_kernels(lib, whe
     check(d(z), d(x), [d(f)], 2.0, beta, d(y), 2.0 ** -24)
 
 
+@pytest.mark.parametrize("option", [8, 16], ids=["TF32", "TF32x3"])
+@pytest.mark.parametrize("P,split", [(127, True), (36, True), (128, None), (64, False)])
+def test_tf32_options_send_what_they_do_not_take_to_the_split_kernel(lib, option, P, split):
+    """A handle with a TF32 option runs the passes that its TF32 kernel declines where a handle without it does."""
+    import torch
+    import fastkron_b200
+    split = option == 16 if split is None else split         # 128x128: TF32 takes it, TF32x3 does not
+    h = fastkron_b200.FastKron()
+    h.set_options(2 | option)
+    M = 4096
+    x, f = torch.rand(M, P, device="cuda") - 0.5, torch.rand(P, P, device="cuda") - 0.5
+    z, t = torch.empty(M, P, device="cuda"), [torch.empty(M * P, device="cuda") for _ in range(2)]
+    n0 = lib.fkbGemmSplitLaunches()
+    h.raw_gemm("mkm", "s", M, [P], [P], x.data_ptr(), 1, [f.data_ptr()], 1, z.data_ptr(), 1.0, 0.0, 0, t[0].data_ptr(), t[1].data_ptr())
+    assert lib.fkbGemmSplitLaunches() - n0 == int(split)
+    if split:
+        d = lambda v: v.cpu().numpy().astype(np.float64)
+        check(d(z), d(x), [d(f)], 1.0, 0.0, None, 2.0 ** -24)
+    h.close()
+
+
 CHAIN = [
     (1, [10] * 5, [10] * 5), (5, [12] * 4, [12] * 4), (300, [5] * 4, [5] * 4), (3, [14, 19, 34, 21], [15, 13, 23, 34]),
     (1, [2] * 9, [2] * 9), (64, [3, 7], [9, 2]), (7, [32, 9, 5], [11, 31, 6]), (2, [1, 6, 1, 5], [3, 1, 2, 4]),
