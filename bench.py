@@ -202,7 +202,7 @@ def time_config(h, c, steps, warmup, profile=False):
         passes = []
         for p in range(per):
             vals = [ms[s * per + p] for s in range(steps)]
-            passes.append({"kind": ["generic", "tile", "gemm", "chain"][kinds[p]], "ms": float(np.mean(vals))})
+            passes.append({"kind": ["generic", "tile", "gemm", "chain", "split"][kinds[p]], "ms": float(np.mean(vals))})
     total_ms = float(sum(times))
     return {"ms_per_step": total_ms / steps, "ms_min": float(min(times)), "launches": int(launches),
             "passes": passes, "buffers": (x, fs, y, z, t1, t2)}
@@ -359,6 +359,8 @@ def workload_desc(c, gpus):
 # matrix (ratio to the algorithmic bytes read), writes are the algorithmic bytes minus what
 # is still dirty in the 126 MB L2 when the kernel ends (an absolute amount, not a ratio).
 NCU_TRAFFIC = {
+    "split": {"read_ratio": 1.0003, "dirty_l2_bytes": 56.4e6,
+              "source": "profiles/gemm_split_kernel.md, passes 2-3: 268.5 MB read, 212.0 MB written for 268.4 MB each way"},
     "gemm": {"read_ratio": 1.0003, "dirty_l2_bytes": 52.8e6,
              "source": "profiles/gemm_kernel_c4_c5.md, C5m passes 2-3: 268.5 MB read, 215.6 MB written for 268.4 MB each way"},
     "tile": {"read_ratio": 1.0002, "dirty_l2_bytes": 50.4e6,
@@ -498,9 +500,7 @@ def dominant_roofline(c, passes, flops, peaks, peak_src, fma_probe, fma_props):
                     "unit": "TFLOP/s", "frac": fp_ach / fp_peak,
                     "peak_source": "larger of the FMA-chain probe of this run (%.1f) and SMs x lanes x 2 x max SM clock "
                                    "from the device properties (%.1f)" % (fma_probe or 0.0, fma_props or 0.0)}, **common)
-    # large fp32 factors run on the tensor cores (exact bf16 splits): the FMA rate bounds nothing there
-    from fastkron_b200 import lib as fk
-    if kind == "gemm" and c["dt"] == "f32" and fk.get().fkbGemmSplitLaunches() > 0:
+    if kind == "split":             # on the tensor cores: the FMA rate bounds nothing there
         return dict(roof_hbm, other=roof_fp)
     return dict(roof_fp, other=roof_hbm) if roof_fp["frac"] > roof_hbm["frac"] else dict(roof_hbm, other=roof_fp)
 

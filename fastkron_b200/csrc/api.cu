@@ -263,7 +263,7 @@ int fkbSetProfiling(fastKronHandle handle, int on) {
   E(handle)->setProfiling(on != 0);
   return 0;
 }
-// Durations (ms) and kernel kinds (0 generic, 1 tile, 2 gemm) of the passes recorded
+// Durations (ms) and kernel kinds (0 generic, 1 tile, 2 gemm, 3 chain, 4 split) of the passes recorded
 // since the last call; synchronises on the recorded events.  Returns the count.
 int fkbGetPassTimes(fastKronHandle handle, float* ms, int* kinds, int maxN) {
   if (!handle || !ms) return -1;

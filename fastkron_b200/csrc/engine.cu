@@ -282,13 +282,13 @@ fastKronError Engine::launchPass(const Pass& ps, const LaunchCtx& cx) {
     evEnd = evPool_[evUsed_ + 1];
     evUsed_ += 2;
   }
-  int ranKind = (int)ps.kind;
+  KernelKind ran = ps.kind;
   fastKronError e = fastKronKernelNotFound;
   if (ps.kind == KernelKind::Tile) e = launchTile(ps, cx);
-  else if (ps.kind == KernelKind::Gemm) e = launchGemm(ps, cx);
+  else if (ps.kind == KernelKind::Gemm) e = launchGemm(ps, cx, &ran);
   else if (ps.kind == KernelKind::Chain) e = launchChain(ps, cx);
-  if (e == fastKronKernelNotFound && ps.nf == 1) { e = launchGeneric(ps, cx); ranKind = (int)KernelKind::Generic; }
-  if (evEnd) { cudaEventRecord(evEnd, stream); evKinds_.push_back(ranKind); }
+  if (e == fastKronKernelNotFound && ps.nf == 1) { e = launchGeneric(ps, cx); ran = KernelKind::Generic; }
+  if (evEnd) { cudaEventRecord(evEnd, stream); evKinds_.push_back((int)ran); }
   if (e != fastKronSuccess) return e;
   gLaunches++;
   return fastKronSuccess;

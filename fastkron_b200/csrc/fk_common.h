@@ -25,7 +25,8 @@ enum class KernelKind : int {
   Generic = 0,   // one thread per output element, arbitrary strides, any P/Q
   Tile    = 1,   // small power-of-two square factors fused in shared memory
   Gemm    = 2,   // large factors, register-blocked FFMA/DFMA contraction
-  Chain   = 3    // several consecutive factors of any shape in one launch
+  Chain   = 3,   // several consecutive factors of any shape in one launch
+  Split   = 4    // not planned: a Gemm pass that ran on the split tensor-core kernel (pass times report it)
 };
 
 // Logical buffer ids a pass reads from / writes to.

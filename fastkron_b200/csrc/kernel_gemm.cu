@@ -111,14 +111,15 @@ static bool fixedForm(const Pass& ps, const LaunchCtx& cx) {
 // The TF32 kernel where a handle asked for it and it takes the pass; then, whatever the handle's options, the split
 // tensor-core kernel where its rule admits the pass, the fixed-shape FMA kernels where they apply, the any-shape kernel
 // otherwise.
-fastKronError launchGemm(const Pass& ps, const LaunchCtx& cx) {
+fastKronError launchGemm(const Pass& ps, const LaunchCtx& cx, KernelKind* ran) {
+  *ran = KernelKind::Gemm;
   const bool fixed = fixedForm(ps, cx);
   if (cx.tf32 && cx.dt == DType::F32 && fixed) {
     const fastKronError e = launchGemmTf32(ps, cx);
     if (e != fastKronKernelNotFound) return e;
   }
   fastKronError e = launchGemmSplit(ps, cx);
-  if (e != fastKronKernelNotFound) return e;
+  if (e != fastKronKernelNotFound) { *ran = KernelKind::Split; return e; }
   if (fixed) {
     e = launchGemmFixed(ps, cx);
     if (e != fastKronKernelNotFound) return e;

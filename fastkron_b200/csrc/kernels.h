@@ -61,7 +61,7 @@ inline bool passBatchCapable(const Pass& ps) {
 fastKronError launchGeneric(const Pass& ps, const LaunchCtx& cx);
 fastKronError launchChain(const Pass& ps, const LaunchCtx& cx);
 fastKronError launchTile(const Pass& ps, const LaunchCtx& cx);
-fastKronError launchGemm(const Pass& ps, const LaunchCtx& cx);
+fastKronError launchGemm(const Pass& ps, const LaunchCtx& cx, KernelKind* ran);   // *ran: Gemm or Split
 fastKronError launchGemmTf32(const Pass& ps, const LaunchCtx& cx);   // only reached through launchGemm
 fastKronError launchGemmSplit(const Pass& ps, const LaunchCtx& cx);  // fp32 on the tensor cores, exact bf16 splits (through launchGemm)
 fastKronError launchGemmAny(const Pass& ps, const LaunchCtx& cx);    // any shape, strides, alignment (through launchGemm)

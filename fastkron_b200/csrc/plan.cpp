@@ -347,7 +347,7 @@ void fuseLaunches(const Problem& pr, const PlanOptions& opt, Plan* plan) {
 
 std::string Plan::describe() const {
   std::ostringstream os;
-  static const char* kn[] = {"generic", "tile", "gemm", "chain"};
+  static const char* kn[] = {"generic", "tile", "gemm", "chain", "split"};
   auto bn = [](Buf b) -> std::string {
     switch (b) { case Buf::X: return "X"; case Buf::T1: return "T1"; case Buf::T2: return "T2";
                  case Buf::Z: return "Z"; default: return "I" + std::to_string((int)b - (int)Buf::I0); }

@@ -273,3 +273,19 @@ def test_bench_host_logic():
     t, src = bench.carried_traffic("gemm", 100e6 * 172, 100e6 * 172)
     assert src.startswith("profiles/") and os.path.exists(os.path.join(ROOT, src.split(",")[0]))
     assert 2 * 100e6 * 172 - 60e6 < t < 2 * 100e6 * 172 + 10e6
+
+
+def test_roofline_entry_follows_the_kernel_that_ran_the_pass():
+    """A pass on the split tensor-core kernel is reported against the copy rate with that kernel's traffic; one on the FMA
+    kernels is not, whatever ran before in the process."""
+    sys.path.insert(0, ROOT)
+    import bench
+    c = {"dt": "f32", "ps": [64] * 4, "M": 256}
+    peaks = {"hbm_gbs": 6400.0}
+    flops = 2 * 256 * 64 ** 5 * 4
+    entry = {}
+    for kind in ("split", "gemm"):
+        entry[kind] = bench.dominant_roofline(c, [{"kind": kind, "ms": 11.0}] * 4, flops, peaks, "test", 72.0, 74.4)
+        assert entry[kind]["kernel"] == kind
+    assert entry["split"]["bound"] == "hbm" and "gemm_split_kernel" in entry["split"]["traffic_source"]
+    assert entry["gemm"]["bound"] == "fp32_simt" and "gemm_kernel_c4_c5" in entry["gemm"]["traffic_source"]
