@@ -1,6 +1,6 @@
 """The split tensor-core pass (csrc/kernel_gemm_split.cu) and the chain launches (csrc/kernel_chain.cu) at the
 sizes where they can go wrong: partial tiles, remainders of 16 and 32, both orientations, operands that are not
-16-byte aligned, beta*Y in place of the result, values that a bf16 split cannot hold.
+16-byte aligned, beta*Y (also in place of the result), batches, streams, values that a bf16 split cannot hold.
 
 Bound.  One step of P products in precision u errs by at most (P + 2) u of the sum of the products' magnitudes
 (one rounding per product for an FMA chain; for the split pass 2.5 u for each 16 products of h*h, a 32nd of that for each of the
@@ -269,6 +269,93 @@ def test_tf32_options_send_what_they_do_not_take_to_the_split_kernel(lib, option
     if split:
         d = lambda v: v.cpu().numpy().astype(np.float64)
         check(d(z), d(x), [d(f)], 1.0, 0.0, None, 2.0 ** -24)
+    h.close()
+
+
+@pytest.mark.parametrize("P,Q,M,runs", [(64, 64, 1023, 0), (64, 64, 1024, 1), (54, 19, 2000, 0), (52, 20, 2000, 1), (16, 64, 2000, 0), (17, 61, 2000, 1),
+                                        (31, 33, 2000, 0), (41, 25, 2000, 1), (128, 128, 1100, 1), (129, 40, 1100, 0), (40, 129, 1100, 0)])
+def test_split_rule_at_its_edges(lib, P, Q, M, runs):
+    """Both sides of every bound of gemmSplitEligible: the kernel that the rule names, the same product."""
+    n0 = lib.fkbGemmSplitLaunches()
+    z, x, fs, y = call("mkm", "f32", M, [P], [Q], 0, 0, 0.0, 0)
+    assert lib.fkbGemmSplitLaunches() - n0 == runs
+    check(z, x, fs, 1.0, 0.0, y, 2.0 ** -24)
+
+
+@pytest.mark.parametrize("P", [64, 128])
+def test_split_pass_in_a_strided_batch(lib, P):
+    """Batches whose entries run one after the other on the split kernel, with factors and Y of their own."""
+    import torch
+    import fastkron_b200
+    h = fastkron_b200.FastKron()
+    batch, M = 3, 1040
+    x, f = torch.rand(batch, M, P, device="cuda") - 0.5, torch.rand(batch, P, P, device="cuda") - 0.5
+    z = torch.rand(batch, M, P, device="cuda")
+    y = z.clone()
+    t = [torch.empty(batch * M * P, device="cuda") for _ in range(2)]
+    n0 = lib.fkbGemmSplitLaunches()
+    h.raw_gemm_strided_batched("mkm", "s", M, [P], [P], x.data_ptr(), 1, M * P, [f.data_ptr()], 1, [P * P], z.data_ptr(), M * P, 2.0, 1.0, batch,
+                               z.data_ptr(), M * P, t[0].data_ptr(), t[1].data_ptr())
+    assert lib.fkbGemmSplitLaunches() == n0 + batch
+    d = lambda v: v.cpu().numpy().astype(np.float64)
+    for b in range(batch):
+        check(d(z[b]), d(x[b]), [d(f[b])], 2.0, 1.0, d(y[b]), 2.0 ** -24)
+    h.close()
+
+
+def test_split_passes_on_two_streams(lib):
+    """Two handles on two streams at once: every CTA takes all of an SM's tensor memory, so the launches take turns on an
+    SM, and the results are those of one after the other."""
+    import torch
+    import fastkron_b200
+    M, P = 6000, 96
+    handles, args = [], []
+    for i in range(2):
+        handles.append(fastkron_b200.FastKron(torch.cuda.Stream()))
+        x, f = torch.rand(M, P, device="cuda") - 0.5, torch.rand(P, P, device="cuda") - 0.5
+        args.append((x, f, torch.empty(M, P, device="cuda"), torch.empty(M * P, device="cuda"), torch.empty(M * P, device="cuda")))
+
+    def go(i):
+        x, f, z, t1, t2 = args[i]
+        handles[i].raw_gemm("mkm", "s", M, [P], [P], x.data_ptr(), 1, [f.data_ptr()], 1, z.data_ptr(), 1.0, 0.0, 0, t1.data_ptr(), t2.data_ptr())
+    torch.cuda.synchronize()
+    for i in range(2):
+        go(i)
+        torch.cuda.synchronize()
+    want = [a[2].clone() for a in args]
+    for a in args:
+        a[2].zero_()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        for i in range(2):
+            go(i)
+    torch.cuda.synchronize()
+    for i in range(2):
+        assert torch.equal(args[i][2], want[i])
+        handles[i].close()
+
+
+@pytest.mark.parametrize("mm", ["mkm", "kmm"])
+@pytest.mark.parametrize("dt", ["f32", "f64"])
+@pytest.mark.parametrize("M,ps,qs", [(40, [12] * 4, [12] * 4), (17, [14, 9], [15, 13]), (5, [10] * 3, [10] * 3)], ids=lambda v: str(v).replace(" ", ""))
+def test_chain_epilogue_in_place(lib, M, ps, qs, dt, mm):
+    """beta*Y with Y in the place of the result."""
+    import torch
+    import fastkron_b200
+    tdt = torch.float32 if dt == "f32" else torch.float64
+    K, L = int(np.prod(ps)), int(np.prod(qs))
+    x, fs = torch.rand(M, K, device="cuda", dtype=tdt) - 0.5, [torch.rand(p, q, device="cuda", dtype=tdt) - 0.5 for p, q in zip(ps, qs)]
+    y = torch.rand(M, L, device="cuda", dtype=tdt)
+    xd, fd, z = (x, fs, y.clone()) if mm == "mkm" else (x.t().contiguous(), [f.t().contiguous() for f in fs], y.t().contiguous())
+    h = fastkron_b200.FastKron()
+    _, te = h.sizes(M, ps, qs)
+    t = [torch.empty(te, device="cuda", dtype=tdt) for _ in range(2)]
+    n0 = lib.fkbLaunchCount()
+    h.raw_gemm(mm, "s" if dt == "f32" else "d", M, ps, qs, xd.data_ptr(), 1, [f.data_ptr() for f in fd], 1, z.data_ptr(), 2.0, -0.5, z.data_ptr(),
+               t[0].data_ptr(), t[1].data_ptr())
+    assert lib.fkbLaunchCount() - n0 < len(ps)
+    d = lambda v: v.cpu().numpy().astype(np.float64)
+    check(d(z if mm == "mkm" else z.t()), d(x), [d(f) for f in fs], 2.0, -0.5, d(y), 2.0 ** -24 if dt == "f32" else 2.0 ** -53)
     h.close()
 
 
