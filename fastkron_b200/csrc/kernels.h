@@ -63,7 +63,7 @@ fastKronError launchChain(const Pass& ps, const LaunchCtx& cx);
 fastKronError launchTile(const Pass& ps, const LaunchCtx& cx);
 fastKronError launchGemm(const Pass& ps, const LaunchCtx& cx, KernelKind* ran);   // *ran: Gemm or Split
 fastKronError launchGemmTf32(const Pass& ps, const LaunchCtx& cx);   // only reached through launchGemm
-fastKronError launchGemmSplit(const Pass& ps, const LaunchCtx& cx);  // fp32 on the tensor cores, exact bf16 splits (through launchGemm)
+fastKronError launchGemmSplit(const Pass& ps, const LaunchCtx& cx);  // fp32 on the tensor cores, bf16 splits (through launchGemm)
 fastKronError launchGemmAny(const Pass& ps, const LaunchCtx& cx);    // any shape, strides, alignment (through launchGemm)
 
 // True when launchTile / launchGemm have an instantiation for the pass; used
